@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(1024) k_cuts_plan(
 }
 
 // K2: local bin of every entry; categorical exact match (unseen -> 0). The
-// histogram codes go to row r at position rpos[f] (rbase[f] + local bin, or
-// rmiss[f] when missing); the feature-major copy holds the local bin itself,
+// histogram codes go to row r at position rpos[f] (rbase[f] + (local bin <<
+// rshift[f]), or rmiss[f] when missing); the feature-major copy holds the local bin itself,
 // MISSING_BIN when missing.
 // The local bin of value v of a feature whose `len` cuts start at `cuts`:
 // bin_of (quantile.rs:166-181), the categorical form an exact match,
@@ -477,12 +477,13 @@ __global__ void __launch_bounds__(BIN_THREADS) k_bin(const float* __restrict__ X
                                              const int* __restrict__ rpos,
                                              const int* __restrict__ rbase,
                                              const int* __restrict__ rmiss,
+                                             const int* __restrict__ rshift,
                                              Code* __restrict__ bins,
                                              uint16_t* __restrict__ bins_col, int sh_cut_cap) {
   extern __shared__ float s_cut[];
   __shared__ uint16_t tl[BIN_TF][BIN_TR + 2];  // local bins [feature][row]
   __shared__ uint32_t s_off[BIN_TF + 1];
-  __shared__ int s_pos[BIN_TF], s_base[BIN_TF], s_miss[BIN_TF];
+  __shared__ int s_pos[BIN_TF], s_base[BIN_TF], s_miss[BIN_TF], s_shift[BIN_TF];
   __shared__ uint8_t s_cat[BIN_TF];
   const bool miss_nan = isnan(missing);
   const int f0 = blockIdx.y * BIN_TF;
@@ -494,6 +495,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_bin(const float* __restrict__ X
     s_pos[i] = rpos[f0 + i];
     s_base[i] = rbase[f0 + i];
     s_miss[i] = rmiss[f0 + i];
+    s_shift[i] = rshift[f0 + i];
     s_cat[i] = is_cat[f0 + i];
   }
   if (sh)
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_bin(const float* __restrict__ X
         const uint16_t local =
             local_bin(v[u], is_missing_d(v[u], missing, miss_nan), cb + s0, s_off[ff + 1] - s0, s_cat[ff] != 0);
         tl[ff][rr] = local;
-        bins[r * Fp + s_pos[ff]] = local == MISSING_BIN ? (Code)s_miss[ff] : (Code)(s_base[ff] + (int)local);
+        bins[r * Fp + s_pos[ff]] = local == MISSING_BIN ? (Code)s_miss[ff] : (Code)(s_base[ff] + ((int)local << s_shift[ff]));
       }
     }
     __syncthreads();
@@ -540,8 +542,6 @@ __global__ void __launch_bounds__(BIN_THREADS) k_bin(const float* __restrict__ X
 
 namespace {
 
-// Indexes with fewer rows take the default layout without timing.
-constexpr size_t TUNE_MIN_ROWS = 200000;
 
 // Shape bucket of the autotuner: device, features, most bins of a feature,
 // log2 of the rows, categorical features present.
@@ -751,12 +751,15 @@ int bin_codes(sb_ctx* ctx, const float* d_X, Ghist* g) {
   DBuf<int>& rpos = g->rpos;
   DBuf<int>& rbase = g->rbase;
   DBuf<int>& rmiss = g->rmiss;
+  DBuf<int>& rshift = g->rshift;
   SB_TRY(rpos.alloc(ctx, F));
   SB_TRY(rbase.alloc(ctx, F));
   SB_TRY(rmiss.alloc(ctx, F));
+  SB_TRY(rshift.alloc(ctx, F));
   SB_CUDA(cudaMemcpyAsync(rpos.p, g->h_rpos.data(), F * 4, cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaMemcpyAsync(rbase.p, g->h_rbase.data(), F * 4, cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaMemcpyAsync(rmiss.p, g->h_rmiss.data(), F * 4, cudaMemcpyHostToDevice, st));
+  SB_CUDA(cudaMemcpyAsync(rshift.p, g->h_rshift.data(), F * 4, cudaMemcpyHostToDevice, st));
   SB_TRY(g->bins_col.alloc(ctx, n * F));
   const size_t rows_per_block = (size_t)BIN_TR * BIN_TILES;
   const dim3 bgrid((unsigned)((n + rows_per_block - 1) / rows_per_block), (unsigned)((F + BIN_TF - 1) / BIN_TF));
@@ -774,13 +777,13 @@ int bin_codes(sb_ctx* ctx, const float* d_X, Ghist* g) {
     SB_TRY(g->bins8.alloc(ctx, n * g->Fp));
     SB_CUDA(cudaMemsetAsync(g->bins8.p, 0xFF, g->bins8.bytes(), st));  // unused positions: 0xFF
     SB_LAUNCH(ctx, k_bin<uint8_t>, bgrid, BIN_THREADS, bsm, d_X, n, (int)F, g->Fp, missing, g->foff.p, g->cuts.p,
-              g->is_cat.p, rpos.p, rbase.p, rmiss.p, g->bins8.p, g->bins_col.p, (int)sh_cuts);
+              g->is_cat.p, rpos.p, rbase.p, rmiss.p, rshift.p, g->bins8.p, g->bins_col.p, (int)sh_cuts);
   } else {
     g->bins8.release();
     SB_TRY(g->bins.alloc(ctx, n * g->Fp));
     SB_CUDA(cudaMemsetAsync(g->bins.p, 0xFF, g->bins.bytes(), st));  // unused positions: 0xFFFF
     SB_LAUNCH(ctx, k_bin<uint16_t>, bgrid, BIN_THREADS, bsm, d_X, n, (int)F, g->Fp, missing, g->foff.p, g->cuts.p,
-              g->is_cat.p, rpos.p, rbase.p, rmiss.p, g->bins.p, g->bins_col.p, (int)sh_cuts);
+              g->is_cat.p, rpos.p, rbase.p, rmiss.p, rshift.p, g->bins.p, g->bins_col.p, (int)sh_cuts);
   }
   SB_CUDA(cudaStreamSynchronize(st));  // the host vectors are released on return
   return SB_OK;

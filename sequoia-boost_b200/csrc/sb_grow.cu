@@ -88,8 +88,9 @@ struct BState {
   const int* fbase;          // code of local bin 0, per feature
   const int* fmiss;          // code of a missing entry, per feature
   const int* rpos;           // row-major codes: position, code of local bin 0 and
-  const int* rbase;          // code of a missing entry of each feature
-  const int* rmiss;
+  const int* rbase;          // code of a missing entry of each feature, and the
+  const int* rmiss;          // shift of its local bins within the code
+  const int* rshift;
   const uint32_t* foff;
   const float* cuts;
   const uint8_t* is_cat;
@@ -1774,7 +1775,7 @@ __global__ void k_lg_route(BState S) {
         bool go;
         if (code == S.rmiss[f]) go = sp.default_left != 0;
         else {
-          const int c = code - S.rbase[f];
+          const int c = (code - S.rbase[f]) >> S.rshift[f];
           go = sp.is_cat ? ((sp.cat_mask[c >> 5] >> (c & 31)) & 1u) != 0 : c <= sp.bin;
         }
         nid = go ? out[nid].left : out[nid].right;
@@ -1880,6 +1881,7 @@ struct sb_booster {
   sb::DBuf<sb::HistItem> d_items;
   sb::DBuf<uint64_t> d_prefix;
   sb::DBuf<int> d_item_count;
+  sb::DBuf<uint64_t> d_parts;
   sb::DBuf<int4> d_ptiles;
   sb::DBuf<int> d_ptile_count;
   sb::DBuf<uint32_t> d_pool, d_upool, d_pool_mask, d_usable;
@@ -2189,6 +2191,7 @@ int booster_init(sb_booster* b, sb_ctx* ctx, const sb_ghist* g, const sb_train_p
   SB_TRY(b->d_items.alloc_zero(ctx, (size_t)K * b->maxw + K));
   SB_TRY(b->d_prefix.alloc_zero(ctx, (size_t)K * b->maxw + K + 1));
   SB_TRY(b->d_item_count.alloc_zero(ctx, 1));
+  SB_TRY(b->d_parts.alloc_zero(ctx, 2 * (size_t)hist_grid(ctx, g, 0, 1)));
   const int ptile_cap = (int)((size_t)K * ((b->n + PART_TILE - 1) / PART_TILE + b->maxn + 1));
   SB_TRY(b->d_ptiles.alloc_zero(ctx, ptile_cap));
   SB_TRY(b->d_ptile_count.alloc_zero(ctx, 1));
@@ -2244,6 +2247,7 @@ int booster_init(sb_booster* b, sb_ctx* ctx, const sb_ghist* g, const sb_train_p
   S.rpos = g->rpos.p;
   S.rbase = g->rbase.p;
   S.rmiss = g->rmiss.p;
+  S.rshift = g->rshift.p;
   S.foff = g->foff.p;
   S.cuts = g->cuts.p;
   S.is_cat = g->is_cat.p;
@@ -2379,10 +2383,11 @@ int booster_round_body(sb_booster* b, int apply_delta) {
   L.rows_done = b->timing ? b->d_hist_rows.p : nullptr;
   L.pool_mask = S.pool_mask;
   L.rows_bound = b->n * (size_t)b->K;  // each class tree's rows at most once per level
+  L.parts = b->d_parts.p;
   const size_t esm = eval_smem(b);
   auto hist = [&](int max_items) -> int {
     L.max_items = max_items;
-    SB_TRY(launch_zero_items(ctx, b->g, S.items, S.item_count, max_items));
+    SB_TRY(launch_zero_items(ctx, L));
     if (b->timing) {
       cudaEvent_t e0, e1;
       SB_CUDA(cudaEventCreate(&e0));
@@ -2686,7 +2691,12 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
     L.rows_done = nullptr;
     L.pool_mask = S.pool_mask;
     L.rows_bound = b->n * (size_t)b->K;
-    L.min_units = 2048;  // the batches' launches overlap: fewer, fuller CTAs for small nodes
+    L.parts = b->d_parts.p;
+    // the batches' launches overlap: fewer, fuller CTAs (64 jobs of 1k-100k
+    // rows, 256-thread CTAs: 512 rows to a CTA and at least 256 units measured
+    // 217 ms of device time per sweep, 1024 / 512 238 ms, 4096 / 2048 254 ms)
+    L.rows_per_cta = 2 * (size_t)b->g->hist_threads;
+    L.min_units = (uint32_t)b->g->hist_threads;
   }
   HistJobsPlan hp;
   SB_TRY(hist_jobs_prepare(ctx, Ls, &hp));
@@ -2836,15 +2846,15 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
 int boosters_train_many(sb_ctx* const* ctxs, int nctx, sb_booster* const* bs, const int* rounds, int nb,
                         int* status) {
   // batchable boosters train in groups that share one histogram kernel: the
-  // same precision, rows per warp instruction and code width
+  // same precision, rows per warp instruction, code width and CTA size
   // (SB_JOBS_BATCH=0: none, every job goes through the stream pool)
   const char* eb = std::getenv("SB_JOBS_BATCH");
   const bool batching = !(eb && std::strcmp(eb, "0") == 0);
-  std::map<std::tuple<int, int, int>, std::vector<int>> groups;
+  std::map<std::tuple<int, int, int, int>, std::vector<int>> groups;
   std::vector<int> rest;
   for (int j = 0; j < nb; ++j) {
     if (status[j] != SB_OK || !bs[j] || rounds[j] <= 0) continue;
-    if (batching && booster_batchable(bs[j])) groups[{bs[j]->S.fixed, bs[j]->g->tiled_rl, bs[j]->g->code_bytes}].push_back(j);
+    if (batching && booster_batchable(bs[j])) groups[{bs[j]->S.fixed, bs[j]->g->tiled_rl, bs[j]->g->code_bytes, bs[j]->g->hist_threads}].push_back(j);
     else rest.push_back(j);
   }
   // a group becomes up to nctx batches of jobs of similar size (each batched

@@ -3,22 +3,21 @@
 // Replaces CpuBackend::build / accumulate (tree/hist/mod.rs:58-119) and
 // `subtracted` / HistogramBackend::subtract (:25-28, :38-44).
 //
-// Design: a persistent grid (one CTA of 1024 threads per SM) splits the
-// concatenated rows of every node to build (all frontier nodes of all class
-// trees in one launch) evenly over CTAs (fewer CTAs for a launch known to
-// hold few rows). A CTA keeps one node's histogram for one feature tile in
-// shared memory, walks its rows in small batches per warp (the low lanes load
-// the row ids ahead and the gradient pairs, shuffles hand them to the warp;
-// TILED keeps two batches in flight), adds every code of a row into the
-// shared partial, and flushes the non-zero entries to the node's HBM
-// histogram with global atomics when it moves to the next piece.
+// Design: a persistent grid (one CTA of 1024 threads per SM, or four of 256
+// where four partials fit) divides the concatenated rows of every node to
+// build (all frontier nodes of all class trees in one launch; cta_parts). A
+// CTA keeps one node's histogram for one feature tile in shared memory, walks
+// its rows with two sub-batches of codes in flight per warp (hist_body), adds
+// every code of a row into the shared partial, and flushes the non-zero
+// entries to the node's HBM histogram with global atomics when it moves to the
+// next piece.
 //   codes  TILED layout: lane l reads features 4l..4l+3 of the tile (one
 //          8-byte load per row) and a code is the entry's index in the tile's
 //          partial, where a feature's bins are contiguous. LANES layout: each
 //          tile gives lane l `S` (1, 2 or 4) code positions of the row, packed
-//          with features so that every lane's entries fit its own column, and
+//          with features so that every lane's entries fit its own column;
 //          entry e of lane l sits at word e * 32 + l: the 32 lanes of a warp
-//          always add into 32 different banks.
+//          add into 32 different banks.
 //   sums   FP32 form: f32 shared atomics, f64 node histograms. FIXED form:
 //          gradients rounded to |q| <= 2^bits with a per-round power-of-two
 //          scale; one int32 and one uint32 shared atomic per entry, exact
@@ -37,16 +36,23 @@ namespace sb {
 namespace {
 
 constexpr int HIST_THREADS = 1024;
+// CTA size where four partials fit one SM (HIST_SMALL_SMEM each): a node of
+// few rows takes a CTA mostly latency (zeroing, the dependent loads of its
+// first rows, flushing), so that four small CTAs per SM take four nodes in the
+// time of one.
+constexpr int HIST_SMALL_THREADS = 256;
+constexpr size_t HIST_SMALL_SMEM = 48 << 10;
 constexpr int MAX_TILE_FEATURES = 128;  // 4 features per lane
-constexpr int ROWS_PER_WARP = 8;        // LANES: rows per warp batch
-constexpr int TILED_ROWS = 4;           // TILED: rows per warp batch (two batches in flight)
+// rows a CTA adds in about the time it zeroes and flushes a partial
+constexpr int FLUSH_ROWS = 1500, FLUSH_ROWS_SMALL = 256;
 
 struct HistDev {
   const uint16_t* bins;  // u16 codes, or null with u8 codes in bins8
   const uint8_t* bins8;
   const uint32_t* foff;
   size_t Fp;             // row stride of bins (u16)
-  const int* ent_gbin;   // LANES: (entry, lane) -> histogram bin, per tile; u8 TILED: entry -> bin
+  const int* rbase;      // LANES: first shared word of each feature, and the shift of its bins
+  const int* rshift;
   const int* slot_feat;  // LANES: feature of each code position of a row
   size_t n;              // gradient column stride
   int total_bins;
@@ -60,8 +66,7 @@ struct HistDev {
   unsigned long long* rows_done;  // sampled rows accumulated (or null)
   const uint32_t* pool_mask;      // [K][FW] features to accumulate (or null: all)
   int FW;
-  int rl;                         // TILED: log2 of the rows one warp instruction covers
-  uint32_t min_units;             // fewest (row, tile) units per active CTA (0: all CTAs)
+  const uint64_t* parts;          // [2 * CTAs] each CTA's part of the rows (cta_parts), or null: equal shares
 };
 
 __device__ __forceinline__ int find_item(const uint64_t* prefix, int count, uint64_t pos) {
@@ -87,41 +92,69 @@ __device__ __forceinline__ void add_pair(unsigned a, unsigned hoff, uint32_t vg,
   }
 }
 
-// The shared partial is two planes of nent 32-bit words, g then h (FIXED:
-// int32 / uint32 integers; FP32: floats), so a warp's atomics spread over all
-// 32 banks. Every entry costs one add into each plane.
-// RL >= 0: the rows per warp instruction (as log2) fixed at compile time;
-// RL < 0: read from the launch description.
-// U8: one-byte codes, the feature's local bin (its bin count when missing);
-// a feature's bins and its missing entry are contiguous in the partial, so an
-// entry's address is the feature's first entry plus the code, and the flush
-// maps entries to histogram bins through the tile's table (ent_gbin).
-template <bool U8> struct CodeWord { using T = uint2; };     // 4 u16 codes
-template <> struct CodeWord<true> { using T = uint32_t; };   // 4 u8 codes
+// Loads of the row gather, volatile so that they stay ahead of the adds they
+// are meant to overlap (the compiler otherwise sinks them towards their use).
+__device__ __forceinline__ uint2 gather(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint16_t gather(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t gather(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
-template <bool FIXED, int RL, bool U8>
-__device__ __forceinline__ void hist_tiled_body(const HistDev& a, unsigned bx, unsigned gdx) {
-  using CW = typename CodeWord<U8>::T;
+// The code layouts of a launch (see sb_internal.cuh): TILED with u16 or u8
+// codes, LANES with 1, 2 or 4 code positions per lane.
+enum { CODES_U16 = 0, CODES_U8 = 1, CODES_LANES1 = 2, CODES_LANES2 = 3, CODES_LANES4 = 4 };
+template <int KIND> struct Codes { using T = uint2; };  // 4 u16 codes
+template <> struct Codes<CODES_U8> { using T = uint32_t; };      // 4 u8 codes
+template <> struct Codes<CODES_LANES1> { using T = uint16_t; };
+template <> struct Codes<CODES_LANES2> { using T = uint32_t; };  // 2 u16 codes
+
+__device__ __forceinline__ uint32_t code_word(const uint2& v, int i) { return i ? v.y : v.x; }
+__device__ __forceinline__ uint32_t code_word(uint32_t v, int) { return v; }
+__device__ __forceinline__ uint32_t code_word(uint16_t v, int) { return v; }
+
+// One CTA's share of a launch. The shared partial is two planes of `words`
+// 32-bit words, g then h (FIXED: int32 / uint32 integers; FP32: floats).
+//
+// What bounds it: the load-store unit. A row costs two shared reductions per
+// code position, a load of its codes and three shuffles, and an instruction
+// whose lanes hit one bank k times takes k passes. So
+//  - the row loop has no predicate or branch at all: a predicated or branched
+//    shared reduction compiles to a branch around it, which also keeps loads
+//    from moving ahead of adds (100 warp instructions per 100-feature row, 45
+//    without; LANES at 10M rows x 100 features, root level, per launch: 756 us
+//    with a test per row, 486 without);
+//  - LANES, whose 32 lanes hit 32 banks, needs 8 passes for 4 positions per
+//    lane where TILED's 25 lanes of random bins need 23.
+template <bool FIXED, int KIND, int RL>
+__device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigned gdx) {
+  constexpr bool LANES = KIND >= CODES_LANES1, U8 = KIND == CODES_U8;
+  constexpr int S = KIND == CODES_LANES1 ? 1 : KIND == CODES_LANES2 ? 2 : 4;  // codes per lane and row
+  constexpr int rl = LANES ? 0 : RL;
+  constexpr int R = rl == 3 ? 2 : S == 4 ? 4 : 8;  // steps per sub-batch
+  constexpr uint32_t SUB = (uint32_t)R << rl;      // rows per sub-batch: two or more fill a block of 32
+  using CW = typename Codes<KIND>::T;
   extern __shared__ unsigned long long sh_u64[];
   unsigned* sh_g = reinterpret_cast<unsigned*>(sh_u64);
   __shared__ double s_tot_d[2];
   __shared__ unsigned long long s_tot_u[2];
 
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int count = *a.count;
   if (count <= 0) return;
   const uint64_t W = a.prefix[count];
   if (W == 0) return;
   const uint64_t U = W * (uint64_t)a.ntiles;
-  // with a.min_units set (batched jobs, whose launches overlap), a launch
-  // holding few rows uses fewer CTAs of at least that many (row, tile) units,
-  // so that zeroing and flushing a shared partial is paid for by enough rows;
-  // the other CTAs return. A lone launch spreads its rows over every CTA.
-  const uint64_t mu = a.min_units ? a.min_units : 1;
-  const uint64_t act = min((uint64_t)gdx, max((uint64_t)1, (U + mu - 1) / mu));
-  if (bx >= act) return;
-  const uint64_t lo = U * bx / act, hi = U * (bx + 1) / act;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-
+  const uint64_t lo = a.parts ? a.parts[2 * bx] : U * bx / gdx, hi = a.parts ? a.parts[2 * bx + 1] : U * (bx + 1) / gdx;
   uint64_t u = lo;
   while (u < hi) {
     const int t = (int)(u / W);
@@ -134,169 +167,227 @@ __device__ __forceinline__ void hist_tiled_body(const HistDev& a, unsigned bx, u
     uint64_t n_pos = piece_hi_u - u;
     if (FIXED && n_pos > a.flush_rows) n_pos = a.flush_rows;
     const uint32_t pbeg = item.begin + (uint32_t)(pos - item_lo);
-    const uint32_t pend = pbeg + (uint32_t)n_pos;
     const FeatureTile tile = a.tiles[t];
     const int nf = tile.f1 - tile.f0;
-    const int nent = tile.nbins + nf;
-    unsigned* sh_h = sh_g + nent;
-    const unsigned sh_base = (unsigned)__cvta_generic_to_shared(sh_g), hoff = 4u * (unsigned)nent;
+    const int nent = LANES ? 32 * tile.E : tile.nbins + nf;  // entries of a plane
+    // words of a plane. LANES: half a bank turn between an entry's g and h, for
+    // the flush. TILED: a word per lane for what is not added; an even count.
+    const int words = LANES ? nent + 16 : (nent + 33) & ~1;
+    unsigned* sh_h = sh_g + words;
+    const unsigned sh_base = (unsigned)__cvta_generic_to_shared(sh_g), hoff = 4u * (unsigned)words;
     const bool want_total = item.root && t == 0;
 
-    // A warp instruction covers 2^rl rows: lane `lane` works on row slot
-    // lane >> (5 - rl) of it and owns the 4 consecutive features
-    // f0 + 4 * grp .. +3 of the tile, grp = its lane within the row's group
-    // (only features of the tree's column pool are added); one 8-byte load
-    // per row fetches their 4 bins. Tiles start at multiples of 4, hold at
-    // most 4 * 32 >> rl features, and rows are padded to a multiple of 8
-    // bins, so the load is aligned and stays inside the row.
-    const int rl = RL >= 0 ? RL : a.rl;
+    // Where the lane's codes of a row sit. TILED: a warp instruction covers
+    // 2^rl rows: the lane works on row slot lane >> (5 - rl) and owns the 4
+    // consecutive features f0 + 4 * grp .. +3 of the tile, grp = its lane
+    // within the row's group (lanes past the tile read its first features and
+    // add none). Tiles start at multiples of 4, hold at most 4 * 32 >> rl
+    // features, and rows are padded to a multiple of 8 codes, so a row's load
+    // is aligned and stays inside it.
     const int grp = lane & ((32 >> rl) - 1), rsub = lane >> (5 - rl);
-    const int fl0 = 4 * grp;
-    const bool lane_on = fl0 < nf;
-    bool fon[4];
-    unsigned eb[4];  // U8: shared address of each owned feature's first entry
+    const bool past = !LANES && 4 * grp >= nf;
+    const int pos0 = LANES ? tile.slot_off + lane * S : tile.f0 + (past ? 0 : 4 * grp);
+    // A code is added at `base` + 4 * code. Positions without a feature of the
+    // tree's pool read as code 0 and add to a word of the lane's own that the
+    // flush leaves out (LANES: entry 0 of its column).
+    unsigned base[S];
+    uint32_t keep[2] = {0, 0};  // code bits that count
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int fl = fl0 + j;
-      const int f = tile.f0 + fl;
-      bool on = fl < nf;
-      eb[j] = sh_base;
-      if (U8 && on) eb[j] = sh_base + 4u * (a.foff[f] - (unsigned)tile.bin0 + (unsigned)fl);
-      if (on && a.pool_mask && !((a.pool_mask[(size_t)item.k * a.FW + (f >> 5)] >> (f & 31)) & 1u)) on = false;
-      fon[j] = on;
+    for (int j = 0; j < S; ++j) {
+      int f = LANES ? a.slot_feat[pos0 + j] : pos0 + j;
+      if (past || (!LANES && f >= tile.f1)) f = -1;
+      const bool in_pool =
+          f >= 0 && (!a.pool_mask || ((a.pool_mask[(size_t)item.k * a.FW + (f >> 5)] >> (f & 31)) & 1u));
+      base[j] = sh_base;
+      if (!in_pool) base[j] += 4u * (unsigned)(LANES ? lane : nent + lane);
+      else if (U8) base[j] += 4u * (a.foff[f] - (unsigned)tile.bin0 + (unsigned)(4 * grp + j));
+      if (in_pool) keep[U8 ? 0 : j >> 1] |= U8 ? 0xFFu << (8 * j) : 0xFFFFu << (16 * (j & 1));
     }
-    for (int i = threadIdx.x; i < 2 * nent; i += blockDim.x) sh_g[i] = 0u;
+    for (int i = threadIdx.x; i < words / 2; i += blockDim.x)
+      reinterpret_cast<uint4*>(sh_g)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < 2) {
       s_tot_d[threadIdx.x] = 0.0;
       s_tot_u[threadIdx.x] = 0ull;
     }
     __syncthreads();
 
-    // Rows go through a warp in batches of TILED_ROWS << rl, double-buffered:
-    // the codes and gradient pairs of the next batch are loaded before the
-    // adds of the current one, so the gather is in flight while the shared
-    // atomics issue. Lane i < the batch size holds row i of a batch (its id,
-    // loaded two batches ahead, and its gradient pair); the other lanes get
-    // them by shuffles. Step q of a batch covers its rows (q << rl) + slot,
-    // and every lane loads its 4 codes of its row.
-    double tg = 0.0, th = 0.0;
-    long long tqg = 0;
-    unsigned long long tqh = 0;
-    unsigned int nsampled = 0;
+    // A warp's rows: FIXED, an equal, contiguous part of the piece; FP32, runs
+    // of RUN rows dealt to the warps in turn, so that the piece's rows are
+    // added in about their own order whatever the load pipeline. They go in
+    // blocks of 32: lane i holds row i of a block, its id loaded two blocks
+    // ahead and its gradient pair one block ahead. The codes are loaded in
+    // sub-batches of SUB rows into two register buffers in turn: the next
+    // sub-batch is requested before the wait for the current one, so that two
+    // are in flight while a warp waits (with one buffer copied to the other,
+    // the copy waited for the newest load: 35 clocks per row instead of 19).
+    // Step q of a sub-batch covers its rows (q << rl) + slot; shuffles hand
+    // every lane its row's id and pair.
     const size_t gcol = (size_t)item.k * a.n;
-    const uint16_t* bins_tile = U8 ? nullptr : a.bins + tile.f0 + fl0;
-    const uint8_t* bins8_tile = U8 ? a.bins8 + tile.f0 + fl0 : nullptr;
-    constexpr int R = TILED_ROWS;
-    const uint32_t B = (uint32_t)R << rl;  // rows per batch (<= 32)
-    const uint32_t stride = (uint32_t)nwarps * B;
-    // the gradient pair of the batch at p (lanes < its rows), counted into the totals
-    auto load_grad = [&](uint32_t rid, uint32_t nr, uint32_t& g, uint32_t& h) {
-      g = 0u;
-      h = 0u;
-      if (lane < (int)nr) {
-        if (FIXED) {
-          const unsigned long long pk = reinterpret_cast<const unsigned long long*>(a.gpair)[gcol + rid];
-          g = (uint32_t)(pk >> 32);
-          h = (uint32_t)(pk & 0xFFFFFFFFull);
-        } else {
-          const float2 v = reinterpret_cast<const float2*>(a.gpair)[gcol + rid];
-          g = __float_as_uint(v.x);
-          h = __float_as_uint(v.y);
+    const CW* codes = reinterpret_cast<const CW*>(U8 ? (const void*)(a.bins8 + pos0) : (const void*)(a.bins + pos0));
+    const uint32_t row_words = (uint32_t)(a.Fp / (U8 ? 4 : S));
+    constexpr uint32_t RUN = LANES ? 8 : 4u << rl;
+    const uint32_t m = (uint32_t)n_pos, per = (m + nwarps - 1) / nwarps, round = nwarps * RUN;
+    const uint32_t p0 = pbeg + (FIXED ? min(m, warp * per) : warp * RUN);
+    const uint32_t nrows = FIXED ? min(m, (warp + 1) * per) - min(m, warp * per)
+                                 : m / round * RUN + min(RUN, max(m % round, warp * RUN) - warp * RUN);
+    // the warp's row v of the piece, in the item's list
+    auto row_at = [&](uint32_t v) { return FIXED ? p0 + v : p0 + v / RUN * round + v % RUN; };
+    double tg = 0.0, th = 0.0;
+    int tqg = 0;  // a piece has at most flush_rows rows of |q| <= 2^bits: 31 bits hold the sums
+    uint32_t tqh = 0;
+    auto load_rid = [&](uint32_t q) { return q + lane < nrows ? item.rows[row_at(q + lane)] : 0u; };
+    auto load_pair = [&](uint32_t q, uint32_t rid, uint32_t& g, uint32_t& h) {
+      uint2 v = make_uint2(0u, 0u);
+      if (q + lane < nrows) v = gather(reinterpret_cast<const uint2*>(a.gpair) + gcol + rid);
+      g = FIXED ? v.y : v.x;  // FIXED: (q_g << 32) + q_h; FP32: {grad, hess}
+      h = FIXED ? v.x : v.y;
+    };
+    // The codes of rows [s, s + SUB) of a block. Positions past the part's end
+    // hold row id 0 and a zero pair: their adds change nothing, and no row
+    // needs a test of its own.
+    auto load_codes = [&](uint32_t rid, uint32_t s, CW (&bv)[R]) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const uint32_t id = __shfl_sync(0xFFFFFFFFu, rid, s + ((uint32_t)q << rl) + (uint32_t)rsub);
+        bv[q] = gather(codes + (uint64_t)id * row_words);
+      }
+    };
+    auto add_codes = [&](uint32_t g, uint32_t h, uint32_t s, const CW (&bv)[R]) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const uint32_t src = s + ((uint32_t)q << rl) + (uint32_t)rsub;
+        const uint32_t vg = __shfl_sync(0xFFFFFFFFu, g, src);
+        const uint32_t vh = __shfl_sync(0xFFFFFFFFu, h, src);
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+          const uint32_t w = code_word(bv[q], U8 ? 0 : j >> 1) & keep[U8 ? 0 : j >> 1];
+          const uint32_t c = U8 ? (w >> (8 * j)) & 0xFFu : (j & 1) ? w >> 16 : w & 0xFFFFu;
+          add_pair<FIXED>(base[j] + 4u * c, hoff, vg, vh);
         }
-        nsampled++;
+      }
+    };
+    if (nrows) {
+      uint32_t p = 0;
+      uint32_t rid_c = load_rid(p), g_c, h_c;
+      uint32_t rid_n = load_rid(p + 32);
+      load_pair(p, rid_c, g_c, h_c);
+      uint32_t nr = min(nrows - p, 32u);
+      CW buf0[R], buf1[R];
+      load_codes(rid_c, 0, buf0);
+      for (;;) {
+        const uint32_t pn = p + 32;
+        const uint32_t nr_n = pn < nrows ? min(nrows - pn, 32u) : 0u;
+        uint32_t g_n, h_n;
+        load_pair(pn, rid_n, g_n, h_n);
+        const uint32_t rid_nn = load_rid(pn + 32);
         if (want_total) {
           if (FIXED) {
-            tqg += (int)g;
-            tqh += h;
+            tqg += (int)g_c;
+            tqh += h_c;
           } else {
-            tg += (double)__uint_as_float(g);
-            th += (double)__uint_as_float(h);
+            tg += (double)__uint_as_float(g_c);
+            th += (double)__uint_as_float(h_c);
           }
         }
-      }
-    };
-    // the codes of the batch's rows (the lists hold sampled rows only)
-    auto load_codes = [&](uint32_t rid, uint32_t nr, CW (&bv)[R]) {
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const uint32_t src = ((uint32_t)q << rl) + (uint32_t)rsub;
-        const uint32_t id = __shfl_sync(0xFFFFFFFFu, rid, src);
-        if constexpr (U8)
-          bv[q] = (src < nr && lane_on) ? __ldg(reinterpret_cast<const uint32_t*>(bins8_tile + (size_t)id * a.Fp)) : 0u;
-        else
-          bv[q] = (src < nr && lane_on) ? __ldg(reinterpret_cast<const uint2*>(bins_tile + (size_t)id * a.Fp))
-                                        : make_uint2(0u, 0u);
-      }
-    };
-    uint32_t p = pbeg + warp * B;
-    uint32_t rid_c = ((uint32_t)lane < B && p + lane < pend) ? item.rows[p + lane] : 0u;
-    uint32_t nrow_c = p < pend ? min(pend - p, B) : 0u;
-    uint32_t g_c, h_c;
-    CW bv_c[R];
-    load_grad(rid_c, nrow_c, g_c, h_c);
-    load_codes(rid_c, nrow_c, bv_c);
-    uint32_t rid_n = ((uint32_t)lane < B && p + stride + lane < pend) ? item.rows[p + stride + lane] : 0u;
-    for (; p < pend; p += stride) {
-      const uint32_t pn = p + stride;
-      const uint32_t nrow_n = pn < pend ? min(pend - pn, B) : 0u;
-      uint32_t g_n, h_n;
-      CW bv_n[R];
-      load_grad(rid_n, nrow_n, g_n, h_n);
-      load_codes(rid_n, nrow_n, bv_n);
-      const uint32_t rid_nn =
-          ((uint32_t)lane < B && pn + stride + lane < pend) ? item.rows[pn + stride + lane] : 0u;
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const uint32_t src = ((uint32_t)q << rl) + (uint32_t)rsub;
-        const uint32_t vg = __shfl_sync(0xFFFFFFFFu, g_c, src);
-        const uint32_t vh = __shfl_sync(0xFFFFFFFFu, h_c, src);
-        if (((uint32_t)q << rl) >= nrow_c) break;  // no row of this step in any lane
-        const bool row_on = src < nrow_c;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          unsigned addr;
-          if constexpr (U8) {
-            addr = eb[j] + 4u * ((bv_c[q] >> (8 * j)) & 0xFFu);  // the feature's entry of the local bin
-          } else {
-            const uint32_t w = j < 2 ? bv_c[q].x : bv_c[q].y;
-            addr = sh_base + 4u * ((j & 1) ? (w >> 16) : (w & 0xFFFFu));  // the tile-relative code
-          }
-          if (fon[j] && row_on) add_pair<FIXED>(addr, hoff, vg, vh);
+#pragma unroll 1
+        for (uint32_t s = 0; s < nr; s += 2 * SUB) {
+          load_codes(rid_c, s + SUB, buf1);
+          add_codes(g_c, h_c, s, buf0);
+          const bool inside = s + 2 * SUB < nr;
+          load_codes(inside ? rid_c : rid_n, inside ? s + 2 * SUB : 0u, buf0);
+          add_codes(g_c, h_c, s + SUB, buf1);
         }
+        if (nr_n == 0) break;
+        p = pn;
+        nr = nr_n;
+        rid_c = rid_n;
+        rid_n = rid_nn;
+        g_c = g_n;
+        h_c = h_n;
       }
-      g_c = g_n;
-      h_c = h_n;
-      nrow_c = nrow_n;
-      rid_n = rid_nn;
-#pragma unroll
-      for (int q = 0; q < R; ++q) bv_c[q] = bv_n[q];
     }
-    if (a.rows_done && t == 0 && nsampled) atomicAdd(a.rows_done, (unsigned long long)nsampled);
-    if (want_total && (uint32_t)lane < B) {  // every lane that held rows of a batch
+    if (a.rows_done && t == 0 && threadIdx.x == 0) atomicAdd(a.rows_done, (unsigned long long)n_pos);
+    if (want_total) {  // one add per warp: 64-bit shared adds to one address go one after another
       if (FIXED) {
-        atomicAdd(&s_tot_u[0], (unsigned long long)tqg);
-        atomicAdd(&s_tot_u[1], tqh);
+        tqg = __reduce_add_sync(0xFFFFFFFFu, tqg);
+        tqh = __reduce_add_sync(0xFFFFFFFFu, tqh);
       } else {
-        atomicAdd(&s_tot_d[0], tg);
-        atomicAdd(&s_tot_d[1], th);
+        for (int o = 16; o > 0; o >>= 1) {
+          tg += __shfl_xor_sync(0xFFFFFFFFu, tg, o);
+          th += __shfl_xor_sync(0xFFFFFFFFu, th, o);
+        }
+      }
+      if (lane == 0) {
+        if (FIXED) {
+          atomicAdd(&s_tot_u[0], (unsigned long long)(long long)tqg);
+          atomicAdd(&s_tot_u[1], (unsigned long long)tqh);
+        } else {
+          atomicAdd(&s_tot_d[0], tg);
+          atomicAdd(&s_tot_d[1], th);
+        }
       }
     }
     __syncthreads();
-    // flush the partial into the node's HBM histogram
-    for (int i = threadIdx.x; i < nent; i += blockDim.x) {
-      const int gi = U8 ? a.ent_gbin[tile.ent_off + i]
-                        : (i < tile.nbins ? tile.bin0 + i : a.total_bins + tile.f0 + (i - tile.nbins));
+    // Flush the partial into the node's HBM histogram, two threads per entry:
+    // a warp's adds then cover whole sectors (570 G words/s over 148 CTAs of
+    // 25,700 entries; g and h in separate instructions 300 G words/s). TILED
+    // u16 entries are in histogram order; the others go one sector of each of
+    // 8 features at a time (LANES: of 8 neighbouring lanes, 2 threads per
+    // bank), their words computed from the feature's place. Four entries per
+    // thread and step keep their shared reads in flight together.
+    unsigned* plane = (lane & 1) ? sh_h : sh_g;
+    auto add_out = [&](int bin, uint32_t v) {
+      const size_t gi = 2 * (size_t)bin + (lane & 1);
+      if (v == 0u) return;
       if (FIXED) {
-        const long long gq = (long long)(int)sh_g[i];
-        const unsigned long long hq = sh_h[i];
-        unsigned long long* o = reinterpret_cast<unsigned long long*>(item.out) + 2 * (size_t)gi;
-        if (gq) atomicAdd(o, (unsigned long long)gq);
-        if (hq) atomicAdd(o + 1, hq);
+        const unsigned long long add =
+            (lane & 1) ? (unsigned long long)v : (unsigned long long)(long long)(int)v;
+        atomicAdd(reinterpret_cast<unsigned long long*>(item.out) + gi, add);
       } else {
-        const float g = __uint_as_float(sh_g[i]), h = __uint_as_float(sh_h[i]);
-        double* o = reinterpret_cast<double*>(item.out) + 2 * (size_t)gi;
-        if (g != 0.0f) atomicAdd(o, (double)g);
-        if (h != 0.0f) atomicAdd(o + 1, (double)h);
+        atomicAdd(reinterpret_cast<double*>(item.out) + gi, (double)__uint_as_float(v));
+      }
+    };
+    if (KIND == CODES_U16) {
+      const int step = blockDim.x >> 1;
+      for (int i0 = threadIdx.x >> 1; i0 < nent; i0 += 4 * step) {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = i0 + j * step < nent ? plane[i0 + j * step] : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = i0 + j * step;
+          add_out(i < tile.nbins ? tile.bin0 + i : a.total_bins + tile.f0 + (i - tile.nbins), v[j]);
+        }
+      }
+    } else {
+      constexpr int CHUNKS = 8;  // warps that share 8 features
+      const int ngroups = LANES ? 4 * S : (nf + 7) / 8, k8 = lane >> 2;
+      for (int unit = warp; unit < ngroups * CHUNKS; unit += nwarps) {
+        const int grp8 = unit / CHUNKS;
+        int f = LANES ? a.slot_feat[tile.slot_off + (8 * (grp8 & 3) + k8) * S + (grp8 >> 2)] : tile.f0 + 8 * grp8 + k8;
+        if (!LANES && f >= tile.f1) f = -1;
+        int first = 0, nb = -1, word = 0, shift = 0;  // nb: the missing entry
+        if (f >= 0) {
+          first = (int)a.foff[f];
+          nb = (int)a.foff[f + 1] - first;
+          word = LANES ? a.rbase[f] : first - tile.bin0 + (f - tile.f0);
+          shift = LANES ? a.rshift[f] : 0;
+        }
+        const int most = __reduce_max_sync(0xFFFFFFFFu, nb);
+        for (int s = unit % CHUNKS; 2 * s - 1 <= most; s += 4 * CHUNKS) {
+          uint32_t v[4];
+          const int b0 = 2 * s + ((lane >> 1) & 1) - (first & 1);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int b = b0 + 2 * CHUNKS * j;
+            v[j] = b >= 0 && b <= nb ? plane[word + (b << shift)] : 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int b = b0 + 2 * CHUNKS * j;
+            add_out(b < nb ? first + b : a.total_bins + f, v[j]);
+          }
+        }
       }
     }
     if (want_total && threadIdx.x == 0) {
@@ -315,9 +406,9 @@ __device__ __forceinline__ void hist_tiled_body(const HistDev& a, unsigned bx, u
   }
 }
 
-template <bool FIXED, int RL, bool U8>
-__global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(HistDev a) {
-  hist_tiled_body<FIXED, RL, U8>(a, blockIdx.x, gridDim.x);
+template <bool FIXED, int KIND, int RL, int THREADS = HIST_THREADS>
+__global__ void __launch_bounds__(THREADS, HIST_THREADS / THREADS) k_hist(HistDev a) {
+  hist_body<FIXED, KIND, RL>(a, blockIdx.x, gridDim.x);
 }
 
 // Many indexes' histogram launches as one (sb_train_many): the x-blocks are
@@ -338,247 +429,137 @@ __device__ __forceinline__ int hist_job_of(const unsigned* xoff, int njobs, unsi
   return lo;
 }
 
-template <bool FIXED, int RL, bool U8>
-__global__ void __launch_bounds__(HIST_THREADS, 1) k_hist_jobs(HistJobs H) {
+template <bool FIXED, int KIND, int RL, int THREADS>
+__global__ void __launch_bounds__(THREADS, HIST_THREADS / THREADS) k_hist_jobs(HistJobs H) {
   const int j = hist_job_of(H.xoff, H.njobs, blockIdx.x);
-  hist_tiled_body<FIXED, RL, U8>(H.devs[j], blockIdx.x - H.xoff[j], H.xoff[j + 1] - H.xoff[j]);
+  __shared__ HistDev s_dev;  // the job's description, as near as a launch's own parameters
+  for (unsigned i = threadIdx.x; i < sizeof(HistDev) / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&s_dev)[i] = reinterpret_cast<const uint32_t*>(H.devs + j)[i];
+  __syncthreads();
+  hist_body<FIXED, KIND, RL>(s_dev, blockIdx.x - H.xoff[j], H.xoff[j + 1] - H.xoff[j]);
 }
 
-template <bool FIXED, bool U8>
-const void* tiled_jobs_pick(int rl) {
+// The TILED kernels for a precision, rows per warp instruction (log2), code
+// width and CTA size: alone, or batched over jobs.
+template <bool FIXED, int KIND, int RL>
+const void* tiled_pick(int threads, bool jobs) {
+  if (threads == HIST_SMALL_THREADS)
+    return jobs ? (const void*)k_hist_jobs<FIXED, KIND, RL, HIST_SMALL_THREADS>
+                : (const void*)k_hist<FIXED, KIND, RL, HIST_SMALL_THREADS>;
+  return jobs ? (const void*)k_hist_jobs<FIXED, KIND, RL, HIST_THREADS> : (const void*)k_hist<FIXED, KIND, RL>;
+}
+template <bool FIXED, int KIND>
+const void* tiled_pick(int rl, int threads, bool jobs) {
   switch (rl) {
-    case 1: return (const void*)k_hist_jobs<FIXED, 1, U8>;
-    case 2: return (const void*)k_hist_jobs<FIXED, 2, U8>;
-    case 3: return (const void*)k_hist_jobs<FIXED, 3, U8>;
-    default: return (const void*)k_hist_jobs<FIXED, 0, U8>;
+    case 1: return tiled_pick<FIXED, KIND, 1>(threads, jobs);
+    case 2: return tiled_pick<FIXED, KIND, 2>(threads, jobs);
+    case 3: return tiled_pick<FIXED, KIND, 3>(threads, jobs);
+    default: return tiled_pick<FIXED, KIND, 0>(threads, jobs);
+  }
+}
+const void* tiled_kernel(bool fixed, const Ghist* g, bool jobs) {
+  const int rl = g->tiled_rl, th = g->hist_threads;
+  if (g->code_bytes == 1) return fixed ? tiled_pick<true, CODES_U8>(rl, th, jobs) : tiled_pick<false, CODES_U8>(rl, th, jobs);
+  return fixed ? tiled_pick<true, CODES_U16>(rl, th, jobs) : tiled_pick<false, CODES_U16>(rl, th, jobs);
+}
+
+const void* lanes_kernel(bool fixed, int slots) {
+  switch (slots) {
+    case 1: return fixed ? (const void*)k_hist<true, CODES_LANES1, 0> : (const void*)k_hist<false, CODES_LANES1, 0>;
+    case 2: return fixed ? (const void*)k_hist<true, CODES_LANES2, 0> : (const void*)k_hist<false, CODES_LANES2, 0>;
+    default: return fixed ? (const void*)k_hist<true, CODES_LANES4, 0> : (const void*)k_hist<false, CODES_LANES4, 0>;
   }
 }
 
-template <bool FIXED, bool U8>
-const void* tiled_pick(int rl) {
-  switch (rl) {
-    case 1: return (const void*)k_hist<FIXED, 1, U8>;
-    case 2: return (const void*)k_hist<FIXED, 2, U8>;
-    case 3: return (const void*)k_hist<FIXED, 3, U8>;
-    default: return (const void*)k_hist<FIXED, 0, U8>;
+// The parts of a launch's CTAs in the tile-major list of (tile, item) row
+// ranges, into parts[2 * CTA] and [2 * CTA + 1]; run by one block of
+// ZERO_THREADS. An equal share of all rows, or, where zeroing and flushing a
+// second partial would cost more than the longer share of whole-range CTAs, a
+// part of one range only: every range gets one CTA and its share of the
+// others. (2M x 200 multiclass lossguide, 20 ranges a launch: 45 us with equal
+// shares, 23 us with one range per CTA.) With min_units set, a launch holding
+// few rows uses fewer CTAs of at least that many (row, tile) units, so that a
+// partial is paid for by enough rows; the others get nothing.
+constexpr int ZERO_THREADS = 256, MAX_RANGES = 1024;
+__device__ void cta_parts(const HistParts& p, int count) {
+  __shared__ uint32_t s_end[MAX_RANGES];  // CTAs of the ranges up to and including each
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint64_t W = count > 0 ? p.prefix[count] : 0, U = W * (uint64_t)p.ntiles;
+  const uint64_t ranges = (uint64_t)max(count, 0) * p.ntiles;
+  const uint64_t mu = p.min_units ? p.min_units : 1;
+  const uint32_t act = (uint32_t)min((uint64_t)p.ctas, max((uint64_t)1, (U + mu - 1) / mu));
+  if (ranges >= act || ranges > MAX_RANGES || U * ranges >= (uint64_t)p.flush_rows * act * (act - ranges)) {
+    for (uint32_t c = tid; c < (uint32_t)p.ctas; c += ZERO_THREADS) {
+      p.parts[2 * c] = c < act ? U * c / act : 0;
+      p.parts[2 * c + 1] = c < act ? U * (c + 1) / act : 0;
+    }
+    return;
+  }
+  const uint32_t nr = (uint32_t)ranges, nc = max(count, 1);
+  for (uint32_t r = tid; r < nr; r += ZERO_THREADS) {  // the CTAs beyond one per range, in proportion, rounded down
+    const uint32_t i = r % nc, len = (uint32_t)(p.prefix[i + 1] - p.prefix[i]);
+    s_end[r] = 1 + (U ? (uint32_t)((double)len * ((double)(act - nr) * (1.0 - 1e-12) / (double)U)) : 0u);
+  }
+  __syncthreads();
+  if (tid < 32) {
+    uint32_t before = 0;
+    for (uint32_t r0 = 0; r0 < nr; r0 += 32) {
+      uint32_t v = r0 + lane < nr ? s_end[r0 + lane] : 0u;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += y;
+      }
+      v += before;
+      if (r0 + lane < nr) s_end[r0 + lane] = v;
+      before = __shfl_sync(0xFFFFFFFFu, v, 31);
+    }
+  }
+  __syncthreads();
+  for (uint32_t c = tid; c < (uint32_t)p.ctas; c += ZERO_THREADS) {
+    uint64_t b = 0, e = 0;
+    if (nr && c < s_end[nr - 1]) {
+      uint32_t lo = 0, hi = nr - 1;  // the first range whose CTAs reach past c
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (s_end[mid] > c) hi = mid; else lo = mid + 1;
+      }
+      const uint32_t c0 = lo ? s_end[lo - 1] : 0u, n = s_end[lo] - c0, q = c - c0;
+      const uint32_t t = lo / nc, i = lo - t * nc;
+      const uint32_t len = (uint32_t)(p.prefix[i + 1] - p.prefix[i]), each = len / n, more = len % n;
+      b = p.prefix[i] + (uint64_t)t * W + (uint64_t)each * q + min(q, more);
+      e = b + each + (q < more ? 1u : 0u);
+    }
+    p.parts[2 * c] = b;
+    p.parts[2 * c + 1] = e;
   }
 }
 
-// The batched TILED kernel for a precision, rows per warp instruction (log2)
-// and code width.
-const void* tiled_jobs_kernel(bool fixed, int rl, bool u8) {
-  if (u8) return fixed ? tiled_jobs_pick<true, true>(rl) : tiled_jobs_pick<false, true>(rl);
-  return fixed ? tiled_jobs_pick<true, false>(rl) : tiled_jobs_pick<false, false>(rl);
-}
-
-// The TILED kernel for a precision, rows per warp instruction (log2) and
-// code width.
-const void* tiled_kernel(bool fixed, int rl, bool u8) {
-  if (u8) return fixed ? tiled_pick<true, true>(rl) : tiled_pick<false, true>(rl);
-  return fixed ? tiled_pick<true, false>(rl) : tiled_pick<false, false>(rl);
-}
-
-// LANES layout (see sb_internal.cuh): lane l of every warp owns the features
-// in its `S` code positions of the tile, and entry e of lane l lives at word
-// e * 32 + l of each plane, so every shared atomic instruction of a warp hits
-// 32 different banks. A row costs one S x u16 load per lane and 2 * S shared
-// atomic instructions per warp; the partial is flushed through the tile's
-// (entry, lane) -> histogram-bin table.
-template <int S> struct Codes;
-template <> struct Codes<1> {
-  using T = unsigned short;
-  __device__ static T none() { return 0xFFFFu; }
-  __device__ static int get(T v, int) { return (int)v; }
-};
-template <> struct Codes<2> {
-  using T = unsigned int;
-  __device__ static T none() { return 0xFFFFFFFFu; }
-  __device__ static int get(T v, int s) { return (int)((v >> (16 * s)) & 0xFFFFu); }
-};
-template <> struct Codes<4> {
-  using T = uint2;
-  __device__ static T none() { return make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu); }
-  __device__ static int get(T v, int s) {
-    const unsigned w = s < 2 ? v.x : v.y;
-    return (int)((w >> (16 * (s & 1))) & 0xFFFFu);
+// Zeroes the node histograms (and root totals) of a launch's items, one grid
+// row per item; the last row divides the rows over the histogram's CTAs.
+__device__ __forceinline__ void zero_items_body(const HistItem* items, const int* count, size_t words,
+                                                const HistParts& parts, unsigned bx, unsigned gdx) {
+  const int it = blockIdx.y, n = *count;
+  if (it == (int)gridDim.y - 1) {
+    if (bx == 0 && parts.parts) cta_parts(parts, n);
+    return;
   }
-};
-
-template <bool FIXED, int S>
-__global__ void __launch_bounds__(HIST_THREADS, 1) k_hist_lanes(HistDev a) {
-  using C = Codes<S>;
-  using CT = typename C::T;
-  extern __shared__ unsigned long long sh_u64[];
-  unsigned* sh_g = reinterpret_cast<unsigned*>(sh_u64);
-  __shared__ double s_tot_d[2];
-  __shared__ unsigned long long s_tot_u[2];
-
-  const int count = *a.count;
-  if (count <= 0) return;
-  const uint64_t W = a.prefix[count];
-  if (W == 0) return;
-  const uint64_t U = W * (uint64_t)a.ntiles;
-  const uint64_t lo = U * blockIdx.x / gridDim.x, hi = U * (blockIdx.x + 1) / gridDim.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-
-  uint64_t u = lo;
-  while (u < hi) {
-    const int t = (int)(u / W);
-    const uint64_t pos = u - (uint64_t)t * W;
-    const int it = find_item(a.prefix, count, pos);
-    const HistItem item = a.items[it];
-    const uint64_t item_lo = a.prefix[it], item_hi = a.prefix[it + 1];
-    uint64_t piece_hi_u = (uint64_t)t * W + item_hi;
-    if (piece_hi_u > hi) piece_hi_u = hi;
-    uint64_t n_pos = piece_hi_u - u;
-    if (FIXED && n_pos > a.flush_rows) n_pos = a.flush_rows;
-    const uint32_t pbeg = item.begin + (uint32_t)(pos - item_lo);
-    const uint32_t pend = pbeg + (uint32_t)n_pos;
-    const FeatureTile tile = a.tiles[t];
-    const int words = 32 * tile.E;  // per plane
-    unsigned* sh_h = sh_g + words;
-    const unsigned sh_base = (unsigned)__cvta_generic_to_shared(sh_g), hoff = 4u * (unsigned)words;
-    const bool want_total = item.root && t == 0;
-
-    // the features of this lane's code positions that the tree's column pool
-    // keeps (unused positions are off)
-    const int slot0 = tile.slot_off + lane * S;
-    bool fon[S];
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const int f = a.slot_feat[slot0 + s];
-      bool on = f >= 0;
-      if (on && a.pool_mask && !((a.pool_mask[(size_t)item.k * a.FW + (f >> 5)] >> (f & 31)) & 1u)) on = false;
-      fon[s] = on;
-    }
-    for (int i = threadIdx.x; i < 2 * words; i += blockDim.x) sh_g[i] = 0u;
-    if (threadIdx.x < 2) {
-      s_tot_d[threadIdx.x] = 0.0;
-      s_tot_u[threadIdx.x] = 0ull;
-    }
-    __syncthreads();
-
-    double tg = 0.0, th = 0.0;
-    long long tqg = 0;
-    unsigned long long tqh = 0;
-    unsigned int nsampled = 0;
-    const size_t gcol = (size_t)item.k * a.n;
-    const uint16_t* bins_lane = a.bins + slot0;
-    const uint32_t stride = (uint32_t)nwarps * ROWS_PER_WARP;
-    uint32_t p = pbeg + warp * ROWS_PER_WARP;
-    uint32_t next_rid = 0u;
-    if (lane < ROWS_PER_WARP && p + lane < pend) next_rid = item.rows[p + lane];
-    for (; p < pend; p += stride) {
-      const uint32_t my_rid = next_rid;
-      const uint32_t pn = p + stride + lane;
-      next_rid = (lane < ROWS_PER_WARP && pn < pend) ? item.rows[pn] : 0u;
-      const uint32_t nrow = min(pend - p, (uint32_t)ROWS_PER_WARP);
-      uint32_t my_g = 0u, my_h = 0u;  // FIXED ints or FP32 float bits
-      if (lane < (int)nrow) {
-        if (FIXED) {
-          const unsigned long long pk = reinterpret_cast<const unsigned long long*>(a.gpair)[gcol + my_rid];
-          my_g = (uint32_t)(pk >> 32);
-          my_h = (uint32_t)(pk & 0xFFFFFFFFull);
-        } else {
-          const float2 v = reinterpret_cast<const float2*>(a.gpair)[gcol + my_rid];
-          my_g = __float_as_uint(v.x);
-          my_h = __float_as_uint(v.y);
-        }
-        nsampled++;
-        if (want_total) {
-          if (FIXED) {
-            tqg += (int)my_g;
-            tqh += my_h;
-          } else {
-            tg += (double)__uint_as_float(my_g);
-            th += (double)__uint_as_float(my_h);
-          }
-        }
-      }
-      CT cv[ROWS_PER_WARP];
-#pragma unroll
-      for (int q = 0; q < ROWS_PER_WARP; ++q) {
-        const uint32_t id = __shfl_sync(0xFFFFFFFFu, my_rid, q);
-        cv[q] = (uint32_t)q < nrow ? __ldg(reinterpret_cast<const CT*>(bins_lane + (size_t)id * a.Fp)) : C::none();
-      }
-#pragma unroll
-      for (int q = 0; q < ROWS_PER_WARP; ++q) {
-        const uint32_t vg = __shfl_sync(0xFFFFFFFFu, my_g, q);
-        const uint32_t vh = __shfl_sync(0xFFFFFFFFu, my_h, q);
-        if ((uint32_t)q >= nrow) break;
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-          if (fon[s]) add_pair<FIXED>(sh_base + 4u * (unsigned)(C::get(cv[q], s) * 32 + lane), hoff, vg, vh);
-      }
-    }
-    if (a.rows_done && t == 0 && nsampled) atomicAdd(a.rows_done, (unsigned long long)nsampled);
-    if (want_total && lane < ROWS_PER_WARP) {
-      if (FIXED) {
-        atomicAdd(&s_tot_u[0], (unsigned long long)tqg);
-        atomicAdd(&s_tot_u[1], tqh);
-      } else {
-        atomicAdd(&s_tot_d[0], tg);
-        atomicAdd(&s_tot_d[1], th);
-      }
-    }
-    __syncthreads();
-    // flush the partial into the node's HBM histogram
-    const int* eg = a.ent_gbin + tile.ent_off;
-    for (int i = threadIdx.x; i < words; i += blockDim.x) {
-      const int gi = eg[i];
-      if (gi < 0) continue;
-      if (FIXED) {
-        const long long gq = (long long)(int)sh_g[i];
-        const unsigned long long hq = sh_h[i];
-        unsigned long long* o = reinterpret_cast<unsigned long long*>(item.out) + 2 * (size_t)gi;
-        if (gq) atomicAdd(o, (unsigned long long)gq);
-        if (hq) atomicAdd(o + 1, hq);
-      } else {
-        const float g = __uint_as_float(sh_g[i]), h = __uint_as_float(sh_h[i]);
-        double* o = reinterpret_cast<double*>(item.out) + 2 * (size_t)gi;
-        if (g != 0.0f) atomicAdd(o, (double)g);
-        if (h != 0.0f) atomicAdd(o + 1, (double)h);
-      }
-    }
-    if (want_total && threadIdx.x == 0) {
-      if (FIXED) {
-        unsigned long long* o = reinterpret_cast<unsigned long long*>(item.total);
-        atomicAdd(o, s_tot_u[0]);
-        atomicAdd(o + 1, s_tot_u[1]);
-      } else {
-        double* o = reinterpret_cast<double*>(item.total);
-        atomicAdd(o, s_tot_d[0]);
-        atomicAdd(o + 1, s_tot_d[1]);
-      }
-    }
-    __syncthreads();
-    u += n_pos;
-  }
-}
-
-__global__ void k_zero_items(const HistItem* __restrict__ items, const int* __restrict__ count,
-                             size_t words) {
-  int it = blockIdx.y;
-  if (it >= *count) return;
+  if (it >= n) return;
   unsigned long long* o = reinterpret_cast<unsigned long long*>(items[it].out);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words;
-       i += (size_t)gridDim.x * blockDim.x)
-    o[i] = 0ull;
-  if (items[it].root && blockIdx.x == 0 && threadIdx.x < 2)
+  for (size_t i = (size_t)bx * blockDim.x + threadIdx.x; i < words; i += (size_t)gdx * blockDim.x) o[i] = 0ull;
+  if (items[it].root && bx == 0 && threadIdx.x < 2)
     reinterpret_cast<unsigned long long*>(items[it].total)[threadIdx.x] = 0ull;
+}
+
+__global__ void k_zero_items(const HistItem* __restrict__ items, const int* __restrict__ count, size_t words,
+                             HistParts parts) {
+  zero_items_body(items, count, words, parts, blockIdx.x, gridDim.x);
 }
 
 // k_zero_items for many jobs: job j's blocks are xoff[j] .. xoff[j + 1] - 1.
 __global__ void k_zero_items_jobs(const ZeroJob* __restrict__ zj, const unsigned* __restrict__ xoff, int njobs) {
   const int j = hist_job_of(xoff, njobs, blockIdx.x);
-  const unsigned bx = blockIdx.x - xoff[j], gdx = xoff[j + 1] - xoff[j];
   const ZeroJob z = zj[j];
-  const int it = blockIdx.y;
-  if (it >= *z.count) return;
-  unsigned long long* o = reinterpret_cast<unsigned long long*>(z.items[it].out);
-  for (size_t i = (size_t)bx * blockDim.x + threadIdx.x; i < z.words; i += (size_t)gdx * blockDim.x) o[i] = 0ull;
-  if (z.items[it].root && bx == 0 && threadIdx.x < 2)
-    reinterpret_cast<unsigned long long*>(z.items[it].total)[threadIdx.x] = 0ull;
+  zero_items_body(z.items, z.count, z.words, z.parts, blockIdx.x - xoff[j], xoff[j + 1] - xoff[j]);
 }
 
 __global__ void k_subtract(const double2* __restrict__ p, const double2* __restrict__ c,
@@ -631,7 +612,7 @@ int plan_tiled(Ghist* g, size_t budget, int rl) {
     size_t f1 = f0;
     while (f1 < F && f1 - f0 < max_tile) {
       size_t bins = g->h_foff[f1 + 1] - g->h_foff[f0];
-      if ((bins + (f1 + 1 - f0)) * 8 > budget) break;
+      if ((bins + (f1 + 1 - f0) + 33) / 2 * 16 > budget) break;
       f1++;
     }
     SB_REQUIRE(f1 > f0, SB_ERR_UNSUPPORTED, "feature %zu has too many bins for shared memory", f0);
@@ -643,7 +624,7 @@ int plan_tiled(Ghist* g, size_t budget, int rl) {
     t.f1 = (int)f1;
     t.bin0 = (int)g->h_foff[f0];
     t.nbins = (int)(g->h_foff[f1] - g->h_foff[f0]);
-    maxb = std::max(maxb, (size_t)(t.nbins + (t.f1 - t.f0)) * 8);
+    maxb = std::max(maxb, (size_t)(t.nbins + (t.f1 - t.f0) + 33) / 2 * 16);
     SB_REQUIRE(t.nbins + (t.f1 - t.f0) < 0xFFFF, SB_ERR_UNSUPPORTED, "histogram tile too large");
     g->tiles.push_back(t);
     f0 = f1;
@@ -660,10 +641,8 @@ int plan_tiled(Ghist* g, size_t budget, int rl) {
   g->h_rpos.assign(F, 0);
   g->h_rbase.assign(F, 0);
   g->h_rmiss.assign(F, 0);
-  int ent_off = 0;
+  g->h_rshift.assign(F, 0);
   for (FeatureTile& t : g->tiles) {
-    t.ent_off = ent_off;
-    ent_off += t.nbins + (t.f1 - t.f0);
     for (int f = t.f0; f < t.f1; ++f) {
       g->h_rpos[f] = f;
       if (g->code_bytes == 1) {  // the local bin; the bin count when missing
@@ -679,31 +658,18 @@ int plan_tiled(Ghist* g, size_t budget, int rl) {
   return SB_OK;
 }
 
-// u8 TILED: the histogram bin of every shared entry, per tile: feature fl of
-// the tile owns entries foff[f] - bin0 + fl .. + its bin count (the last one
-// its missing entry, bin total_bins + f).
-std::vector<int> tiled_u8_entries(const Ghist* g) {
-  std::vector<int> eg;
-  for (const FeatureTile& t : g->tiles) {
-    eg.resize((size_t)t.ent_off + t.nbins + (t.f1 - t.f0), -1);
-    for (int f = t.f0; f < t.f1; ++f) {
-      const int nb = (int)(g->h_foff[f + 1] - g->h_foff[f]);
-      const size_t e0 = (size_t)t.ent_off + (g->h_foff[f] - t.bin0) + (f - t.f0);
-      for (int b = 0; b < nb; ++b) eg[e0 + b] = (int)g->h_foff[f] + b;
-      eg[e0 + nb] = (int)(g->total_bins + f);
-    }
-  }
-  return eg;
-}
-
-// One feature's place in the LANES layout.
+// One feature's place in the LANES layout: bin b at shared word
+// word + (b << shift) (shift 5 in the lane's own column, else 0).
 struct LanePlace {
-  int lane, slot, eb;  // lane, code position within the lane, first entry
+  int lane, slot, word, shift;
 };
 
 // Longest-processing-time packing of features [f0, f1) into 32 lanes of
-// `slots` positions with at most `emax` entries (bins + the missing entry)
-// per lane. Returns the largest lane load, or -1 when the features do not fit.
+// `slots` positions, at most `emax` rows of 32 words. Row 0 of every lane's
+// column takes what is not a feature's. Features whose bins fit no column any
+// more (the fourth 257-bin feature of a lane) get consecutive words in rows
+// below the columns: a few lanes' adds to random banks cost less than another
+// tile. Returns the rows used, or -1 when the features do not fit.
 int pack_lanes(const Ghist* g, size_t f0, size_t f1, int slots, int emax, std::vector<LanePlace>* out) {
   const size_t m = f1 - f0;
   if (m > (size_t)32 * slots) return -1;
@@ -711,62 +677,73 @@ int pack_lanes(const Ghist* g, size_t f0, size_t f1, int slots, int emax, std::v
   for (size_t i = 0; i < m; ++i) order[i] = (int)(f0 + i);
   auto ent = [&](int f) { return (int)(g->h_foff[f + 1] - g->h_foff[f]) + 1; };
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ent(a) > ent(b); });
-  int load[32] = {0}, used[32] = {0};
-  out->assign(m, LanePlace{0, 0, 0});
-  int emx = 1;
-  for (int f : order) {
-    int best = -1;
-    for (int l = 0; l < 32; ++l)
-      if (used[l] < slots && (best < 0 || load[l] < load[best])) best = l;
-    if (best < 0 || load[best] + ent(f) > emax) return -1;
-    (*out)[f - f0] = LanePlace{best, used[best]++, load[best]};
-    load[best] += ent(f);
-    emx = std::max(emx, load[best]);
+  for (int reserve = 0;;) {  // rows kept for the features outside the columns
+    int load[32], used[32] = {0};
+    for (int& l : load) l = 1;
+    out->assign(m, LanePlace{0, 0, 0, 5});
+    std::vector<int> rest;
+    int rows = 1, rest_words = 0;
+    for (int f : order) {
+      int best = -1;
+      for (int l = 0; l < 32; ++l)
+        if (used[l] < slots && (best < 0 || load[l] < load[best])) best = l;
+      if (best < 0 || load[best] + ent(f) > emax - reserve) {
+        rest.push_back(f);
+        rest_words += ent(f);
+        continue;
+      }
+      (*out)[f - f0] = LanePlace{best, used[best]++, load[best] * 32 + best, 5};
+      load[best] += ent(f);
+      rows = std::max(rows, load[best]);
+    }
+    const int rest_rows = (rest_words + 31) / 32;
+    if (rows + rest_rows <= emax) {
+      int word = rows * 32;
+      for (int f : rest) {
+        const int l = (int)(std::min_element(used, used + 32) - used);
+        (*out)[f - f0] = LanePlace{l, used[l]++, word, 0};
+        word += ent(f);
+      }
+      return rows + rest_rows;
+    }
+    if (rest_rows <= reserve) return -1;
+    reserve = rest_rows;
   }
-  return emx;
 }
 
-// LANES layout: tiles grow feature by feature while their features still pack
-// into the 32 lanes.
+// LANES layout: the fewest tiles of near-equal feature counts whose features
+// all pack into the 32 lanes (a last tile of few features would cost a pass
+// over the rows of its own).
 int plan_lanes(Ghist* g, size_t budget, int slots, std::vector<std::vector<LanePlace>>* places) {
   const size_t F = g->F;
-  const int emax = (int)std::min<size_t>(budget / (2 * 32 * 4), 0xFFFE);
-  std::vector<FeatureTile> tiles;
-  places->clear();
-  size_t f0 = 0;
-  int ent_off = 0;
-  std::vector<LanePlace> cur, best;
-  while (f0 < F) {
-    size_t f1 = f0;
-    int E = -1;
-    while (f1 < F) {
-      int e = pack_lanes(g, f0, f1 + 1, slots, emax, &cur);
-      if (e < 0) break;
-      E = e;
-      best = cur;
-      f1++;
+  const int emax = (int)std::min<size_t>((budget / 8 - 16) / 32, 0xFFFF / 32);
+  for (size_t T = (F + 32 * slots - 1) / (32 * slots); T <= F; ++T) {
+    std::vector<FeatureTile> tiles;
+    places->clear();
+    for (size_t i = 0; i < T; ++i) {
+      FeatureTile t{};
+      t.f0 = (int)(F * i / T);
+      t.f1 = (int)(F * (i + 1) / T);
+      std::vector<LanePlace> at;
+      t.E = pack_lanes(g, t.f0, t.f1, slots, emax, &at);
+      if (t.E < 0) break;
+      t.bin0 = (int)g->h_foff[t.f0];
+      t.nbins = (int)(g->h_foff[t.f1] - g->h_foff[t.f0]);
+      t.slot_off = (int)i * 32 * slots;
+      tiles.push_back(t);
+      places->push_back(at);
     }
-    if (f1 == f0) return SB_ERR_UNSUPPORTED;  // one feature's bins exceed a lane
-    FeatureTile t{};
-    t.f0 = (int)f0;
-    t.f1 = (int)f1;
-    t.bin0 = (int)g->h_foff[f0];
-    t.nbins = (int)(g->h_foff[f1] - g->h_foff[f0]);
-    t.E = E;
-    t.ent_off = ent_off;
-    t.slot_off = (int)tiles.size() * 32 * slots;
-    ent_off += 32 * E;
-    tiles.push_back(t);
-    places->push_back(best);
-    f0 = f1;
+    if (tiles.size() == T) {
+      g->tiles = tiles;
+      return SB_OK;
+    }
   }
-  g->tiles = tiles;
-  return SB_OK;
+  return SB_ERR_UNSUPPORTED;  // one feature's bins exceed the partial
 }
 
 size_t lanes_smem(const Ghist* g) {
   size_t m = 0;
-  for (const FeatureTile& t : g->tiles) m = std::max(m, (size_t)t.E * 32 * 4 * 2);
+  for (const FeatureTile& t : g->tiles) m = std::max(m, ((size_t)t.E * 32 + 16) * 8);
   return m;
 }
 
@@ -789,12 +766,6 @@ int hist_prepare(sb_ctx* ctx, Ghist* g, HistChoice c) {
   const size_t F = g->F;
   if (c.layout == HIST_LAYOUT_TILED) {
     SB_TRY(plan_tiled(g, budget, c.rl));
-    if (g->code_bytes == 1) {
-      const std::vector<int> eg = tiled_u8_entries(g);
-      SB_TRY(g->ent_gbin.alloc(ctx, eg.size()));
-      SB_CUDA(cudaMemcpyAsync(g->ent_gbin.p, eg.data(), eg.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-      SB_CUDA(cudaStreamSynchronize(ctx->stream));  // the pageable copy must finish before eg goes away
-    }
   } else {
     const int slots = c.slots;
     SB_REQUIRE(slots == 1 || slots == 2 || slots == 4, SB_ERR_INVALID_ARG, "internal: %d slots", slots);
@@ -808,69 +779,60 @@ int hist_prepare(sb_ctx* ctx, Ghist* g, HistChoice c) {
     g->h_rpos.assign(F, 0);
     g->h_rbase.assign(F, 0);
     g->h_rmiss.assign(F, 0);
-    size_t ent_total = 0;
-    for (const FeatureTile& t : g->tiles) ent_total += (size_t)32 * t.E;
-    std::vector<int> eg(ent_total, -1), sf(g->Fp, -1);
+    g->h_rshift.assign(F, 0);
+    std::vector<int> sf(g->Fp, -1);
     for (size_t ti = 0; ti < g->tiles.size(); ++ti) {
       const FeatureTile& t = g->tiles[ti];
       for (int f = t.f0; f < t.f1; ++f) {
         const LanePlace& pl = places[ti][f - t.f0];
-        const int nb = (int)(g->h_foff[f + 1] - g->h_foff[f]);
         g->h_rpos[f] = t.slot_off + pl.lane * slots + pl.slot;
-        g->h_rbase[f] = pl.eb;
-        g->h_rmiss[f] = pl.eb + nb;
+        g->h_rbase[f] = pl.word;
+        g->h_rshift[f] = pl.shift;
+        g->h_rmiss[f] = pl.word + ((int)(g->h_foff[f + 1] - g->h_foff[f]) << pl.shift);
         sf[g->h_rpos[f]] = f;
-        for (int b = 0; b < nb; ++b) eg[t.ent_off + (size_t)(pl.eb + b) * 32 + pl.lane] = (int)g->h_foff[f] + b;
-        eg[t.ent_off + (size_t)(pl.eb + nb) * 32 + pl.lane] = (int)(g->total_bins + f);
       }
     }
-    SB_TRY(g->ent_gbin.alloc(ctx, eg.size()));
     SB_TRY(g->slot_feat.alloc(ctx, sf.size()));
-    SB_CUDA(cudaMemcpyAsync(g->ent_gbin.p, eg.data(), eg.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
     SB_CUDA(cudaMemcpyAsync(g->slot_feat.p, sf.data(), sf.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    // the pageable copies above must finish before the vectors go away
-    SB_CUDA(cudaStreamSynchronize(ctx->stream));
+    SB_CUDA(cudaStreamSynchronize(ctx->stream));  // the pageable copy must finish before sf goes away
     g->hist_smem_bytes = lanes_smem(g);
   }
+  g->hist_threads =
+      g->layout == HIST_LAYOUT_TILED && g->hist_smem_bytes <= HIST_SMALL_SMEM ? HIST_SMALL_THREADS : HIST_THREADS;
+  if (g->layout == HIST_LAYOUT_TILED)
+    for (int fixed = 0; fixed < 2; ++fixed) SB_TRY(raise_smem_limit(tiled_kernel(fixed != 0, g, false), g->hist_smem_bytes));
   for (int fixed = 0; fixed < 2; ++fixed)
-    for (int rl = 0; rl < 4; ++rl)
-      for (int u8 = 0; u8 < 2; ++u8) SB_TRY(raise_smem_limit(tiled_kernel(fixed != 0, rl, u8 != 0), g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<false, 1>, g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<true, 1>, g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<false, 2>, g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<true, 2>, g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<false, 4>, g->hist_smem_bytes));
-  SB_TRY(raise_smem_limit((const void*)k_hist_lanes<true, 4>, g->hist_smem_bytes));
+    for (int slots : {1, 2, 4}) SB_TRY(raise_smem_limit(lanes_kernel(fixed != 0, slots), g->hist_smem_bytes));
   return SB_OK;
 }
 
-// The layout an index takes without timing: TILED, or what SB_HIST_LAYOUT
-// ("tiled" or "lanes") in the environment forces. On the 10M x 100 binary
-// workload TILED measured 0.41 ms per histogram launch against 0.48 ms for
-// LANES with 4 positions per lane, so LANES is only chosen by timing.
+// The layout an index takes without timing, or what SB_HIST_LAYOUT ("tiled"
+// or "lanes") in the environment forces. Wide matrices (more than 64 features)
+// of 200k rows and more take LANES with 4 positions per lane where it packs:
+// its adds never meet in a bank. Measured per launch, root / deepest level, us:
+// 10M x 100 x 256 bins 481 / 255 against TILED's 955 / 403; 300k x 100 48 / 80
+// against 71 / 79; 3M x 70 x 64 bins (TILED u8) 141 / 72 against 252 / 115.
+// Smaller indexes take TILED, the layout that batched jobs share.
 int hist_default_choice(sb_ctx* ctx, Ghist* g, HistChoice* out) {
   const size_t F = g->F;
   const char* force = std::getenv("SB_HIST_LAYOUT");
   const bool force_lanes = force && std::strcmp(force, "lanes") == 0;
   *out = HistChoice{HIST_LAYOUT_TILED, 0};
-  if (!force_lanes) return SB_OK;
+  if (!force_lanes && (force || std::getenv("SB_HIST_ROWS") || F <= 64 || g->n < TUNE_MIN_ROWS)) return SB_OK;
   const int slots = F <= 32 ? 1 : (F <= 64 ? 2 : 4);
   std::vector<std::vector<LanePlace>> places;
   const std::vector<FeatureTile> keep = g->tiles;
   const bool ok = plan_lanes(g, smem_budget(ctx), slots, &places) == SB_OK;
   g->tiles = keep;
-  SB_REQUIRE(ok, SB_ERR_UNSUPPORTED, "SB_HIST_LAYOUT=lanes: a feature has too many bins");
-  *out = HistChoice{HIST_LAYOUT_LANES, slots};
+  SB_REQUIRE(ok || !force_lanes, SB_ERR_UNSUPPORTED, "SB_HIST_LAYOUT=lanes: a feature has too many bins");
+  if (ok) *out = HistChoice{HIST_LAYOUT_LANES, slots};
   return SB_OK;
 }
 
-// The choices the autotuner times: TILED, and for up to 64 features (where
-// one row per warp instruction keeps at most 16 of a warp's lanes busy)
-// TILED with 2, 4 or 8 rows per instruction and LANES with 1 and 2 positions
-// per lane where the features pack. Wider matrices take TILED: on
-// the 10M x 100 workload a whole round measured TILED faster at every level
-// (ncu: LANES cut the shared-atomic wavefronts by 2.4x but waited longer on
-// its 23 % longer rows), while a single timed launch ranked LANES first.
+// The choices the autotuner times for up to 64 features: TILED with 1, 2, 4
+// or 8 rows per instruction (one row per instruction keeps at most 16 of a
+// warp's lanes busy) and LANES with 1 and 2 positions per lane where the
+// features pack. Wider matrices take hist_default_choice's rule.
 std::vector<HistChoice> hist_candidates(sb_ctx* ctx, Ghist* g) {
   std::vector<HistChoice> out{HistChoice{HIST_LAYOUT_TILED, 0, 0}};
   if (g->F > 64) return out;
@@ -890,31 +852,23 @@ std::vector<HistChoice> hist_candidates(sb_ctx* ctx, Ghist* g) {
 namespace {
 
 const void* hist_kernel(const Ghist* g, bool fixed) {
-  if (g->layout == HIST_LAYOUT_LANES) {
-    switch (g->slots) {
-      case 1: return fixed ? (const void*)k_hist_lanes<true, 1> : (const void*)k_hist_lanes<false, 1>;
-      case 2: return fixed ? (const void*)k_hist_lanes<true, 2> : (const void*)k_hist_lanes<false, 2>;
-      default: return fixed ? (const void*)k_hist_lanes<true, 4> : (const void*)k_hist_lanes<false, 4>;
-    }
-  }
-  return tiled_kernel(fixed, g->tiled_rl, g->code_bytes == 1);
+  if (g->layout == HIST_LAYOUT_LANES) return lanes_kernel(fixed, g->slots);
+  return tiled_kernel(fixed, g, false);
 }
 
 }  // namespace
 
-// The persistent grid: every resident CTA, or for a launch known to hold
-// few rows one CTA per HIST_MIN_ROWS_PER_CTA (row, tile) units, so that a
-// small job's launch zeroes and flushes few shared partials and leaves SMs
-// to the launches of other streams.
-constexpr size_t HIST_MIN_ROWS_PER_CTA = 4096;
-int hist_grid(sb_ctx* ctx, const Ghist* g, size_t rows_bound) {
+// The persistent grid: every resident CTA, or for a launch known to hold few
+// rows one CTA per `rows_per_cta` (row, tile) units (a batched job leaves SMs
+// to the other batches' launches).
+int hist_grid(sb_ctx* ctx, const Ghist* g, size_t rows_bound, size_t rows_per_cta) {
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist_kernel(g, true), HIST_THREADS,
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist_kernel(g, true), g->hist_threads,
                                                 g->hist_smem_bytes);
   if (per_sm < 1) per_sm = 1;
   const size_t full = (size_t)ctx->num_sms * per_sm;
   if (rows_bound == 0) return (int)full;
-  const size_t want = (rows_bound * g->tiles.size() + HIST_MIN_ROWS_PER_CTA - 1) / HIST_MIN_ROWS_PER_CTA;
+  const size_t want = (rows_bound * g->tiles.size() + rows_per_cta - 1) / rows_per_cta;
   return (int)std::max<size_t>(1, std::min(full, want));
 }
 
@@ -925,7 +879,8 @@ static HistDev hist_dev(const HistLaunch& L) {
   a.bins8 = L.g->code_bytes == 1 ? L.g->bins8.p : nullptr;
   a.foff = L.g->foff.p;
   a.Fp = L.g->Fp;
-  a.ent_gbin = L.g->ent_gbin.p;
+  a.rbase = L.g->rbase.p;
+  a.rshift = L.g->rshift.p;
   a.slot_feat = L.g->slot_feat.p;
   a.n = L.g->n;
   a.total_bins = (int)L.g->total_bins;
@@ -939,34 +894,36 @@ static HistDev hist_dev(const HistLaunch& L) {
   a.rows_done = L.rows_done;
   a.pool_mask = L.pool_mask;
   a.FW = (int)((L.g->F + 31) / 32);
-  a.rl = L.g->tiled_rl;
-  a.min_units = L.min_units;
+  a.parts = L.parts;
   return a;
 }
 
 int launch_hist(sb_ctx* ctx, const HistLaunch& L) {
   const HistDev a = hist_dev(L);
-  const int grid = hist_grid(ctx, L.g, L.rows_bound);
+  const int grid = hist_grid(ctx, L.g, L.rows_bound, L.rows_per_cta);
   const size_t sm = L.g->hist_smem_bytes;
-  void (*kern)(HistDev) = reinterpret_cast<void (*)(HistDev)>(
-      const_cast<void*>(tiled_kernel(L.fixed, L.g->tiled_rl, L.g->code_bytes == 1)));
-  if (L.g->layout == HIST_LAYOUT_LANES) {
-    switch (L.g->slots) {
-      case 1: kern = L.fixed ? k_hist_lanes<true, 1> : k_hist_lanes<false, 1>; break;
-      case 2: kern = L.fixed ? k_hist_lanes<true, 2> : k_hist_lanes<false, 2>; break;
-      default: kern = L.fixed ? k_hist_lanes<true, 4> : k_hist_lanes<false, 4>;
-    }
-  }
-  SB_LAUNCH(ctx, kern, grid, HIST_THREADS, sm, a);
+  void (*kern)(HistDev) = reinterpret_cast<void (*)(HistDev)>(const_cast<void*>(hist_kernel(L.g, L.fixed != 0)));
+  SB_LAUNCH(ctx, kern, grid, L.g->hist_threads, sm, a);
   return SB_OK;
 }
 
-int launch_zero_items(sb_ctx* ctx, const Ghist* g, const HistItem* items, const int* count,
-                      int max_items) {
-  if (max_items <= 0) return SB_OK;
-  size_t words = (g->total_bins + g->F) * 2;
-  dim3 grid((unsigned)std::min<size_t>((words + 255) / 256, 64), (unsigned)max_items);
-  SB_LAUNCH(ctx, k_zero_items, grid, 256, 0, items, count, words);
+// The division of a launch's rows over its CTAs (cta_parts).
+static HistParts hist_parts(sb_ctx* ctx, const HistLaunch& L) {
+  HistParts p;
+  p.prefix = L.prefix;
+  p.ntiles = L.ntiles;
+  p.ctas = hist_grid(ctx, L.g, L.rows_bound, L.rows_per_cta);
+  p.min_units = L.min_units;
+  p.flush_rows = L.g->hist_threads == HIST_SMALL_THREADS ? FLUSH_ROWS_SMALL : FLUSH_ROWS;
+  p.parts = L.parts;
+  return p;
+}
+
+int launch_zero_items(sb_ctx* ctx, const HistLaunch& L) {
+  if (L.max_items <= 0) return SB_OK;
+  const size_t words = (L.g->total_bins + L.g->F) * 2;
+  dim3 grid((unsigned)std::min<size_t>((words + 255) / 256, 64), (unsigned)L.max_items + 1);
+  SB_LAUNCH(ctx, k_zero_items, grid, ZERO_THREADS, 0, L.items, L.count, words, hist_parts(ctx, L));
   return SB_OK;
 }
 
@@ -982,14 +939,14 @@ int hist_jobs_prepare(sb_ctx* ctx, const std::vector<HistLaunch>& Ls, HistJobsPl
   for (int j = 0; j < nj; ++j) {
     const HistLaunch& L = Ls[j];
     SB_REQUIRE(L.g->layout == HIST_LAYOUT_TILED && L.fixed == P->fixed && L.g->tiled_rl == Ls[0].g->tiled_rl &&
-                   L.g->code_bytes == Ls[0].g->code_bytes,
+                   L.g->code_bytes == Ls[0].g->code_bytes && L.g->hist_threads == Ls[0].g->hist_threads,
                SB_ERR_INVALID_ARG,
-               "internal: batched histograms need the TILED layout, one precision, one row grouping and one "
-               "code width");
+               "internal: batched histograms need the TILED layout, one precision, one row grouping, one "
+               "code width and one CTA size");
     devs[j] = hist_dev(L);
     const size_t words = (L.g->total_bins + L.g->F) * 2;
-    zero[j] = ZeroJob{L.items, L.count, words};
-    P->hist_grid[j] = (unsigned)hist_grid(ctx, L.g, L.rows_bound);
+    zero[j] = ZeroJob{L.items, L.count, words, hist_parts(ctx, L)};
+    P->hist_grid[j] = (unsigned)hist_grid(ctx, L.g, L.rows_bound, L.rows_per_cta);
     P->zero_grid[j] = (unsigned)std::min<size_t>((words + 255) / 256, 64);
     P->smem = std::max(P->smem, L.g->hist_smem_bytes);
   }
@@ -999,9 +956,9 @@ int hist_jobs_prepare(sb_ctx* ctx, const std::vector<HistLaunch>& Ls, HistJobsPl
   SB_TRY(P->zero.alloc(ctx, nj));
   SB_CUDA(cudaMemcpyAsync(P->devs.p, devs.data(), nj * sizeof(HistDev), cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaMemcpyAsync(P->zero.p, zero.data(), nj * sizeof(ZeroJob), cudaMemcpyHostToDevice, st));
-  P->rl = Ls[0].g->tiled_rl;
-  P->u8 = Ls[0].g->code_bytes == 1;
-  SB_TRY(raise_smem_limit(tiled_jobs_kernel(P->fixed != 0, P->rl, P->u8), P->smem));
+  P->kernel = tiled_kernel(P->fixed != 0, Ls[0].g, true);
+  P->threads = Ls[0].g->hist_threads;
+  SB_TRY(raise_smem_limit(P->kernel, P->smem));
   SB_CUDA(cudaStreamSynchronize(st));  // the host tables are released on return
   return SB_OK;
 }
@@ -1009,14 +966,14 @@ int hist_jobs_prepare(sb_ctx* ctx, const std::vector<HistLaunch>& Ls, HistJobsPl
 int launch_hist_jobs(sb_ctx* ctx, const HistJobsPlan& P, const unsigned* d_xoff, unsigned hist_blocks,
                      const unsigned* d_zoff, unsigned zero_blocks, int max_items) {
   if (max_items <= 0 || hist_blocks == 0) return SB_OK;
-  SB_LAUNCH(ctx, k_zero_items_jobs, dim3(zero_blocks, (unsigned)max_items), 256, 0, P.zero.p, d_zoff, P.njobs);
+  SB_LAUNCH(ctx, k_zero_items_jobs, dim3(zero_blocks, (unsigned)max_items + 1), ZERO_THREADS, 0, P.zero.p, d_zoff, P.njobs);
   HistJobs H;
   H.devs = reinterpret_cast<const HistDev*>(P.devs.p);
   H.xoff = d_xoff;
   H.njobs = P.njobs;
   void (*kern)(HistJobs) =
-      reinterpret_cast<void (*)(HistJobs)>(const_cast<void*>(tiled_jobs_kernel(P.fixed != 0, P.rl, P.u8)));
-  SB_LAUNCH(ctx, kern, hist_blocks, HIST_THREADS, P.smem, H);
+      reinterpret_cast<void (*)(HistJobs)>(const_cast<void*>(P.kernel));
+  SB_LAUNCH(ctx, kern, hist_blocks, P.threads, P.smem, H);
   return SB_OK;
 }
 

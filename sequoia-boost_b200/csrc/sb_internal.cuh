@@ -122,9 +122,10 @@ constexpr uint32_t UNSAMPLED = 0x80000000u;  // row-list flag: not in the subset
 //         holds each feature's bins followed by its missing entry.
 //  LANES: each tile gives each of the 32 lanes of a warp `slots` code
 //         positions (row stride Fp = tiles * 32 * slots); lane l owns the
-//         features placed in its slots, and the code is the entry's index e
-//         in lane l's own column of the partial, stored at word e * 32 + l,
-//         so the 32 lanes of a warp always add into 32 different banks.
+//         features placed in its slots, the code is a word of the partial, and
+//         entry e of lane l sits at word e * 32 + l, so the 32 lanes of a warp
+//         add into 32 different banks (but for features outside the columns,
+//         see pack_lanes).
 enum { HIST_LAYOUT_TILED = 0, HIST_LAYOUT_LANES = 1 };
 
 // A feature tile of the histogram: features [f0, f1), whose entries fit in the
@@ -133,10 +134,8 @@ struct FeatureTile {
   int f0, f1;
   int bin0;       // foff[f0]
   int nbins;      // foff[f1] - foff[f0]
-  int E;          // LANES: entries per lane (the partial has 32 * E words per plane)
-  int ent_off;    // LANES, u8 TILED: offset of the tile's entry -> histogram-bin table
+  int E;          // LANES: rows of the partial (32 * E words per plane)
   int slot_off;   // LANES: position of the tile's first code in a row
-  int reserved;
 };
 
 struct Ghist {  // sb_ghist
@@ -154,16 +153,14 @@ struct Ghist {  // sb_ghist
   // feature's bins and its missing entry fit a byte (at most 255 bins), else 2.
   int code_bytes = 2;
   // [n][Fp] bin codes of the histogram kernel: feature f of row r at
-  // r * Fp + rpos[f], code = rbase[f] + local bin, or rmiss[f] for a missing
-  // entry; unused positions hold 0xFFFF (0xFF). `bins` holds u16 codes,
-  // `bins8` u8 codes (rbase 0, rmiss the feature's bin count); only the one
-  // of `code_bytes` is allocated.
+  // r * Fp + rpos[f], code = rbase[f] + (local bin << rshift[f]), or rmiss[f]
+  // for a missing entry; unused positions hold 0xFFFF (0xFF). `bins` holds u16
+  // codes, `bins8` u8 codes (rbase 0, rmiss the feature's bin count); only the
+  // one of `code_bytes` is allocated.
   DBuf<uint16_t> bins;
   DBuf<uint8_t> bins8;
-  std::vector<int> h_rpos, h_rbase, h_rmiss;
-  DBuf<int> rpos, rbase, rmiss;  // device copies of h_rpos, h_rbase, h_rmiss
-  DBuf<int> ent_gbin;      // LANES: per tile, [E][32] histogram bin of each (entry, lane), -1 unused;
-                           // u8 TILED: per tile, the histogram bin of each shared entry
+  std::vector<int> h_rpos, h_rbase, h_rmiss, h_rshift;
+  DBuf<int> rpos, rbase, rmiss, rshift;  // device copies of the above
   DBuf<int> slot_feat;     // LANES: [Fp] feature of each code position, -1 unused
   // [F][n] local bins, feature-major, MISSING_BIN for a missing entry (the
   // partition reads them): code = fbase[f] + local, fmiss[f] when missing
@@ -178,6 +175,7 @@ struct Ghist {  // sb_ghist
   std::vector<uint8_t> h_is_cat;
   std::vector<FeatureTile> tiles;  // histogram feature tiles
   size_t hist_smem_bytes = 0;      // shared memory of the largest tile
+  int hist_threads = 0;            // CTA size of the histogram kernel
 };
 
 // A binned matrix lives on the device of the context that built it; an entry
@@ -228,7 +226,17 @@ struct HistLaunch {
   unsigned long long* rows_done;  // device counter of sampled rows, or null
   const uint32_t* pool_mask;      // device [K][ceil(F/32)]: features to accumulate, or null
   size_t rows_bound = 0;          // most rows one launch accumulates (0: unknown, full grid)
+  size_t rows_per_cta = 128;      // (row, tile) units per CTA of a launch with few rows (hist_grid)
   uint32_t min_units = 0;         // fewest (row, tile) units per active CTA (0: every CTA works)
+  uint64_t* parts = nullptr;      // device [2 * hist_grid]: filled by launch_zero_items, or null: equal shares
+};
+
+// How a launch's rows are divided over its CTAs.
+struct HistParts {
+  const uint64_t* prefix;
+  int ntiles, ctas;
+  uint32_t min_units, flush_rows;
+  uint64_t* parts;
 };
 
 // Zeroing of one job's node histograms in a batched launch.
@@ -236,6 +244,7 @@ struct ZeroJob {
   const HistItem* items;
   const int* count;
   size_t words;  // 64-bit words per node histogram
+  HistParts parts;
 };
 
 // Device tables of histogram launches over many jobs (sb_train_many): job j
@@ -249,8 +258,8 @@ struct HistJobsPlan {
   std::vector<unsigned> hist_grid, zero_grid;
   int njobs = 0;
   int fixed = 0;
-  int rl = 0;  // rows per warp instruction (log2), the same for every job
-  bool u8 = false;  // one-byte codes, the same for every job
+  const void* kernel = nullptr;  // the jobs' histogram kernel: one row grouping, code width and CTA size
+  int threads = 0;
   size_t smem = 0;
 };
 int hist_jobs_prepare(sb_ctx* ctx, const std::vector<HistLaunch>& Ls, HistJobsPlan* P);
@@ -266,14 +275,15 @@ struct HistChoice {
   int slots;
   int rl = -1;  // TILED: rows per warp instruction (log2); -1: by the feature count
 };
+// Indexes with fewer rows take the TILED layout without timing.
+constexpr size_t TUNE_MIN_ROWS = 200000;
 int hist_prepare(sb_ctx* ctx, Ghist* g, HistChoice c);
 int hist_default_choice(sb_ctx* ctx, Ghist* g, HistChoice* out);
 std::vector<HistChoice> hist_candidates(sb_ctx* ctx, Ghist* g);
 int hist_time(sb_ctx* ctx, const Ghist* g, float* ms);
 int launch_hist(sb_ctx* ctx, const HistLaunch& L);
-int launch_zero_items(sb_ctx* ctx, const Ghist* g, const HistItem* items, const int* count,
-                      int max_items);
-int hist_grid(sb_ctx* ctx, const Ghist* g, size_t rows_bound);
+int launch_zero_items(sb_ctx* ctx, const HistLaunch& L);  // before launch_hist: zeroes L's items, fills L.parts
+int hist_grid(sb_ctx* ctx, const Ghist* g, size_t rows_bound, size_t rows_per_cta);
 // Depthwise boosters that can share batched round launches (no lossguide,
 // external gradients, timing, eval sets or row -> leaf output; TILED index).
 bool booster_batchable(const sb_booster* b);
