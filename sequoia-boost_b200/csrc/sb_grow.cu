@@ -15,7 +15,7 @@
 // One boosting round is a fixed sequence of kernels whose work sizes live in
 // device memory (no host round trip inside a round):
 //   k_gradient -> k_round_prep -> [k_quantize] -> root histograms ->
-//   per level d: k_eval_scan -> k_eval_pick -> k_assign -> k_partition -> k_plan -> histograms
+//   per level d: k_eval -> k_assign -> k_partition -> k_plan -> histograms
 //   -> k_round_end.
 // All frontier nodes of all K class trees are processed by each launch.
 #include <algorithm>
@@ -57,6 +57,7 @@ struct __align__(8) Fill {
 };
 
 struct FeatRec;
+struct FeatBest;
 
 // An entry of a lossguide tree's priority queue (NodeEntry ordered by
 // loss_chg.total_cmp, hist.rs:79-95).
@@ -161,7 +162,8 @@ struct BState {
   int4* ptiles;
   int* ptile_count;
   int ptile_cap;
-  FeatRec* frec;            // [K][maxw][F] phase-2a summaries
+  FeatRec* frec;            // [K][maxw][F] the features' records
+  FeatBest* fbest;          // [K][maxw][F] the best candidates, by pool position
   // sampling
   uint32_t* pool;           // [K][F] the tree's colsample_bytree pool, ascending
   int* pool_len;            // [K]
@@ -170,7 +172,8 @@ struct BState {
   uint32_t* pool_mask;      // [K][FW] bitmask of upool
   const uint32_t* usable;   // [FW] features with >= 2 bins
   uint32_t* samp_scratch;   // [max(1024, K)][F] when per-node sampling is on
-  double* mbuf;             // [K][maxw][F] phase-1 best gain per (node, feature)
+  double* mbuf;             // [K][maxw][F] best gain per node and pool position
+  unsigned* eval_done;      // [K][maxw] finished eval blocks of a node (0 between launches)
   // outputs
   sb_node* out_nodes;       // [tree_cap][maxn]
   uint32_t* out_cats;       // [tree_cap][cat_cap]
@@ -653,11 +656,12 @@ struct EvalNode {
 };
 
 __device__ __forceinline__ double2 hist_entry(const BState& S, const char* H, int i, int k) {
+  // from L2: the last block of a node reads what other blocks of the launch wrote
   if (S.fixed) {
-    longlong2 q = reinterpret_cast<const longlong2*>(H)[i];
+    longlong2 q = __ldcg(reinterpret_cast<const longlong2*>(H) + i);
     return make_double2(dmul((double)q.x, S.inv_scale[2 * k]), dmul((double)q.y, S.inv_scale[2 * k + 1]));
   }
-  return reinterpret_cast<const double2*>(H)[i];
+  return __ldcg(reinterpret_cast<const double2*>(H) + i);
 }
 
 // Gain of one candidate (consider, hist.rs:549-596). -inf when the candidate
@@ -734,7 +738,7 @@ __device__ __forceinline__ CatScratch cat_scratch(double* base, int warp, int ca
 
 constexpr int AMB_MAX = 6;  // ambiguous records kept per (node, feature)
 
-// Phase-2 summary of one feature of one node (see k_eval_records).
+// The records of one feature of one node (see k_eval_body).
 struct FeatRec {
   double def_gain;          // gain of the last certain record
   int def_idx;              // its candidate index, -1 none
@@ -745,7 +749,8 @@ struct FeatRec {
 
 struct Chosen {
   double gain;
-  int cand;    // candidate index within the feature, -1 none
+  int cand;       // candidate index within the feature, -1 none
+  double before;  // SCAN_MAX: best gain of the earlier candidates
 };
 
 enum { SCAN_MAX = 0, SCAN_REPLAY = 1, SCAN_RECORDS = 2, SCAN_EXTRACT = 3 };
@@ -757,7 +762,8 @@ enum { SCAN_MAX = 0, SCAN_REPLAY = 1, SCAN_RECORDS = 2, SCAN_EXTRACT = 3 };
 //   category : prefixes of the non-empty bins sorted by G/(H+lambda)
 //              (evaluate_categorical, hist.rs:607-653); candidate index = prefix
 // Modes:
-//   SCAN_MAX     the feature's best candidate gain
+//   SCAN_MAX     the feature's best candidate gain, the first candidate with it
+//                and the best gain before that one
 //   SCAN_RECORDS with the prefix maximum P started at `b_in` (the best gain of
 //                earlier features, or 0): the last candidate with g > P + eps
 //                (certainly taken by consider's rule g > best + 1e-6) and the
@@ -818,7 +824,7 @@ __device__ Chosen scan_feature(const BState& S, const char* H, int k, int f, con
     __syncwarp();
     ncand = nne - 1;  // prefixes leaving at least one category right
   }
-  Chosen res{MODE == SCAN_MAX ? -INFINITY : b_in, -1};
+  Chosen res{MODE == SCAN_MAX ? -INFINITY : b_in, -1, -INFINITY};
   if (ncand <= 0) {
     if (MODE == SCAN_RECORDS && lane == 0) {
       rec->def_idx = -1;
@@ -827,8 +833,7 @@ __device__ Chosen scan_feature(const BState& S, const char* H, int k, int f, con
     return res;
   }
 
-  double run_max = -INFINITY;  // SCAN_MAX
-  double P = b_in;             // prefix maximum (RECORDS / REPLAY)
+  double P = MODE == SCAN_MAX ? -INFINITY : b_in;  // prefix maximum
   int def_idx = -1;            // RECORDS: last certain record
   double def_gain = 0.0;
   int namb = 0;                // RECORDS: ambiguous records after def_idx (lane 0's copy)
@@ -859,7 +864,15 @@ __device__ Chosen scan_feature(const BState& S, const char* H, int k, int f, con
     }
     const double lm = fmax(gA, gB);
     if (MODE == SCAN_MAX) {
-      run_max = fmax(run_max, lm);
+      const double top = warp_max(lm);
+      if (top > P) {
+        const int owner = __ffs(__ballot_sync(0xFFFFFFFFu, lm == top)) - 1;
+        const double PA = warp_excl_max(lm, P);  // best before candidate 2i (or i)
+        const bool isB = gB > gA;
+        res.before = __shfl_sync(0xFFFFFFFFu, fmax(P, isB ? fmax(PA, gA) : PA), owner);
+        res.cand = cat ? c0 + owner : 2 * (c0 + owner) + __shfl_sync(0xFFFFFFFFu, (int)isB, owner);
+        P = top;
+      }
     } else if (MODE == SCAN_EXTRACT) {
       if (out && (want >> (cat ? 0 : 1)) == i) {
         const bool isB = !cat && (want & 1);
@@ -942,7 +955,7 @@ __device__ Chosen scan_feature(const BState& S, const char* H, int k, int f, con
     cg += tg;
     ch += th;
   }
-  if (MODE == SCAN_MAX) res.gain = warp_max(run_max);
+  if (MODE == SCAN_MAX) res.gain = P;
   if (MODE == SCAN_RECORDS && lane == 0) {
     rec->def_idx = def_idx;
     rec->def_gain = def_gain;
@@ -996,149 +1009,517 @@ constexpr int SCAN_WARPS = EVAL_THREADS / 32;
 
 __device__ __forceinline__ bool in_mask(const uint32_t* m, int f) { return (m[f >> 5] >> (f & 31)) & 1u; }
 
-// Phase 1, one warp per (frontier node, usable pool feature): materialise the
-// feature's bins of a node whose histogram is the parent's minus the built
-// sibling's (the subtraction trick, K5), then record the feature's best
-// candidate gain (-inf when the node may not use the feature).
-__device__ __forceinline__ void k_eval_scan_body(const BState& S, unsigned bx, unsigned gdx, int d) {
-  extern __shared__ double ev_sm[];
+// A numeric feature of up to NUM_BINS bins: its bins go to shared memory with
+// coalesced loads, lane l takes an odd number `e` of consecutive ones (odd:
+// the 16-byte accesses of 8 lanes then hit 8 bank groups), and one warp scan
+// of the lanes' totals turns them into prefix sums in place. The sums are the
+// same in any order (FIXED: integers times a power of two, exact in f64), and
+// the candidates' gains are independent of one another, where 32 bins at a
+// time had a chain of nine scans.
+constexpr int LANE_BINS = 9, NUM_BINS = 32 * LANE_BINS;
+
+struct NumScan {
+  const double2* sum;  // prefix sums (shared)
+  double2 miss;        // the missing bin
+  double pg, ph;       // all bins
+  int e, nb;           // bins per lane; bins
+};
+
+// The per-warp share of the eval kernel's dynamic shared memory.
+__host__ __device__ constexpr size_t eval_warp_bytes(int cat_bins) {
+  const size_t num = (size_t)NUM_BINS * 16, cat = (cat_scratch_bytes(cat_bins) + 15) / 16 * 16;
+  return cat > num ? cat : num;
+}
+
+// Feature f's prefix sums into `sm` (NUM_BINS entries). With P and B set, the
+// bins are P's less B's and are also stored to H.
+__device__ __forceinline__ void num_load(const BState& S, char* H, const char* P, const char* B, int k, int f,
+                                         double2* sm, NumScan* N) {
+  const int lane = threadIdx.x & 31;
+  const int fs = (int)S.foff[f], nb = (int)S.foff[f + 1] - fs;
+  const double sg = S.fixed ? S.inv_scale[2 * k] : 1.0, sh = S.fixed ? S.inv_scale[2 * k + 1] : 1.0;
+  longlong2 x[LANE_BINS + 1], y[LANE_BINS + 1];  // bit patterns of double2 for FP32
+  auto at = [&](int c) { return c < LANE_BINS ? fs + c * 32 + lane : S.total_bins + f; };
+  auto in = [&](int c) { return c < LANE_BINS ? c * 32 + lane < nb : true; };
+  const longlong2* src = reinterpret_cast<const longlong2*>(P ? P : H);
+#pragma unroll
+  for (int c = 0; c <= LANE_BINS; ++c) x[c] = in(c) ? __ldcg(src + at(c)) : make_longlong2(0, 0);
+  if (P) {
+#pragma unroll
+    for (int c = 0; c <= LANE_BINS; ++c)
+      y[c] = in(c) ? __ldcg(reinterpret_cast<const longlong2*>(B) + at(c)) : make_longlong2(0, 0);
+#pragma unroll
+    for (int c = 0; c <= LANE_BINS; ++c) {
+      if (!in(c)) continue;
+      if (S.fixed) {
+        x[c] = make_longlong2(x[c].x - y[c].x, x[c].y - y[c].y);
+      } else {
+        x[c].x = __double_as_longlong(dsub(__longlong_as_double(x[c].x), __longlong_as_double(y[c].x)));
+        x[c].y = __double_as_longlong(dsub(__longlong_as_double(x[c].y), __longlong_as_double(y[c].y)));
+      }
+      if (c < LANE_BINS || lane == 0) reinterpret_cast<longlong2*>(H)[at(c)] = x[c];
+    }
+  }
+  auto value = [&](const longlong2& q) {
+    return S.fixed ? make_double2(dmul((double)q.x, sg), dmul((double)q.y, sh))
+                   : make_double2(__longlong_as_double(q.x), __longlong_as_double(q.y));
+  };
+  __syncwarp();  // the last use of `sm`
+#pragma unroll
+  for (int c = 0; c < LANE_BINS; ++c)
+    if (c * 32 < nb) sm[c * 32 + lane] = value(x[c]);
+  N->miss = value(x[LANE_BINS]);
+  __syncwarp();
+  N->sum = sm;
+  N->nb = nb;
+  N->e = (nb + 31) / 32 | 1;
+  const int i0 = lane * N->e, i1 = min(nb, i0 + N->e);
+  double g = 0.0, h = 0.0;
+  for (int i = i0; i < i1; ++i) {
+    const double2 v = sm[i];
+    g = dadd(g, v.x);
+    h = dadd(h, v.y);
+  }
+  const double ig = warp_incl_sum(g), ih = warp_incl_sum(h);
+  N->pg = __shfl_sync(0xFFFFFFFFu, ig, 31);
+  N->ph = __shfl_sync(0xFFFFFFFFu, ih, 31);
+  g = __shfl_up_sync(0xFFFFFFFFu, ig, 1);
+  h = __shfl_up_sync(0xFFFFFFFFu, ih, 1);
+  if (lane == 0) g = h = 0.0;
+  for (int i = i0; i < i1; ++i) {
+    const double2 v = sm[i];
+    g = dadd(g, v.x);
+    h = dadd(h, v.y);
+    sm[i] = make_double2(g, h);
+  }
+  __syncwarp();
+}
+
+// Left and right sums of candidate c (2 * bin + direction): .x, .y of each.
+__device__ __forceinline__ void num_sides(const NumScan& N, const EvalNode& E, int c, double2* l, double2* r) {
+  const double2 a = N.sum[c >> 1];
+  if (c & 1) {  // missing left
+    *l = make_double2(dadd(a.x, N.miss.x), dadd(a.y, N.miss.y));
+    *r = make_double2(dsub(N.pg, a.x), dsub(N.ph, a.y));
+  } else {
+    *l = a;
+    *r = make_double2(dsub(E.tg, a.x), dsub(E.th, a.y));
+  }
+}
+
+__device__ __forceinline__ double num_gain(const BState& S, const NumScan& N, const EvalNode& E, int dir, int c) {
+  if ((c >> 1) >= N.nb - 1 || ((c & 1) && !(N.miss.y > 1e-6))) return -INFINITY;
+  double2 l, r;
+  double wl, wr;
+  num_sides(N, E, c, &l, &r);
+  return cand_gain(S, E, dir, l.x, l.y, r.x, r.y, &wl, &wr);
+}
+
+// One side's part of a candidate's gain (calc_gain, or gain_at_weight at the
+// bounded weight) with 1 / (h + lambda) to a relative error of about 2^-39: a
+// reciprocal of 20 bits and one Newton step. It only screens: what it lets
+// through is evaluated with divisions. *w is the weight, *size what the error
+// is relative to.
+constexpr double SCREEN_ERR = 1.0 / (1 << 30);
+__device__ __forceinline__ double screen_side(const BState& S, const EvalNode& E, double g, double h, double* w,
+                                              double* size) {
+  const double t = threshold_l1(g, S.reg.alpha), b = dadd(h, S.reg.lambda);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  if (!S.constrained && S.reg.mds == 0.0) {
+    *w = 0.0;
+    return *size = h <= 0.0 ? 0.0 : dmul(dmul(t, t), r);
+  }
+  double a = h <= 0.0 ? 0.0 : dmul(-t, r);
+  if (S.reg.mds > 0.0) a = clampd(a, -S.reg.mds, S.reg.mds);
+  if (S.constrained) a = clampd(a, E.lo, E.hi);
+  *w = a;
+  if (h <= 0.0) return *size = 0.0;
+  const double u = dmul(dmul(2.0, t), a), v = dmul(dmul(b, a), a);
+  *size = dadd(fabs(u), v);
+  return -dadd(u, v);
+}
+
+// The best candidate of a numeric feature: its gain, its sums, its index (the
+// first with that gain), and whether no earlier candidate comes within
+// CLEAR of it. Candidates are screened by bounds on their gains, and only
+// those that can be the best are evaluated with divisions (a division is some
+// forty instructions and a branch; a feature has up to 576 candidates and one
+// or two that come near its best).
+constexpr double CLEAR = 2e-3;
+struct __align__(16) FeatBest {
+  double lg, lh, rg, rh;
+  int idx;
+  int clear;
+  int feature;
+  int sums;  // lg .. rh are filled in
+};
+__device__ __forceinline__ double num_best(const BState& S, const NumScan& N, const EvalNode& E, int f,
+                                           FeatBest* out) {
+  const int lane = threadIdx.x & 31, dir = S.mono ? S.mono[f] : 0;
+  const bool both = N.miss.y > 1e-6;
+  float ub[2 * LANE_BINS];
+  double lb = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < 2 * LANE_BINS; ++c) {
+    ub[c] = -INFINITY;
+    const int i = lane * N.e + (c >> 1);
+    if ((c >> 1) >= N.e || i >= N.nb - 1 || ((c & 1) && !both)) continue;
+    double2 l, r;
+    num_sides(N, E, 2 * i + (c & 1), &l, &r);
+    if (!(l.y >= S.reg.mcw && r.y >= S.reg.mcw)) continue;
+    double wl, wr, sl, sr;
+    const double t = dadd(screen_side(S, E, l.x, l.y, &wl, &sl), screen_side(S, E, r.x, r.y, &wr, &sr));
+    const double err = dmul(SCREEN_ERR, dadd(dadd(sl, sr), fabs(E.parent_gain)));
+    const double v = dsub(t, E.parent_gain);
+    bool sure = true;
+    if (S.constrained && dir) {  // satisfies(dir, wl, wr), or too near to say
+      const double by = dir > 0 ? dsub(wr, wl) : dsub(wl, wr), margin = dmul(SCREEN_ERR, dadd(fabs(wl), fabs(wr)));
+      if (by < -margin) continue;
+      sure = by > margin;
+    }
+    ub[c] = __double2float_ru(dadd(v, err));
+    if (sure) lb = fmax(lb, dsub(v, err));
+  }
+  lb = warp_max(lb);
+  uint32_t todo = 0;
+#pragma unroll
+  for (int c = 0; c < 2 * LANE_BINS; ++c)
+    if (ub[c] != -INFINITY && !((double)ub[c] < lb)) todo |= 1u << c;  // NaN bounds are evaluated
+  double best = -INFINITY;
+  int at = 0x7FFFFFFF;
+  while (__any_sync(0xFFFFFFFFu, todo != 0)) {
+    if (todo) {
+      const int c = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const double g = num_gain(S, N, E, dir, 2 * lane * N.e + c);
+      if (g > best) {
+        best = g;
+        at = 2 * lane * N.e + c;
+      }
+    }
+  }
+  const double M = warp_max(best);
+  int m = best == M ? at : 0x7FFFFFFF;
+  for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  bool near = false;
+#pragma unroll
+  for (int c = 0; c < 2 * LANE_BINS; ++c)
+    near |= 2 * lane * N.e + c < m && ub[c] != -INFINITY && !((double)ub[c] < dsub(M, CLEAR));
+  const bool any_near = __any_sync(0xFFFFFFFFu, near);
+  if (m != 0x7FFFFFFF && lane == 0) {
+    double2 l, r;
+    num_sides(N, E, m, &l, &r);
+    *out = FeatBest{l.x, l.y, r.x, r.y, m, any_near ? 0 : 1, f, 1};
+  } else if (lane == 0) {
+    out->clear = 0;
+  }
+  return M;
+}
+
+// SCAN_RECORDS of scan_feature for a numeric feature in registers.
+__device__ __forceinline__ void num_records(const BState& S, const NumScan& N, const EvalNode& E, int f, double q,
+                                            FeatRec* rec) {
+  const int lane = threadIdx.x & 31, dir = S.mono ? S.mono[f] : 0;
+  double g[2 * LANE_BINS], top = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < LANE_BINS; ++j) {
+    g[2 * j] = j < N.e ? num_gain(S, N, E, dir, 2 * (lane * N.e + j)) : -INFINITY;
+    g[2 * j + 1] = j < N.e ? num_gain(S, N, E, dir, 2 * (lane * N.e + j) + 1) : -INFINITY;
+    top = fmax(top, fmax(g[2 * j], g[2 * j + 1]));
+  }
+  // the lane's candidates in order, from the best of the earlier lanes and q
+  double P = warp_excl_max(top, q);
+  int last = -1;
+  double last_gain = 0.0;
+  uint32_t amb = 0;  // ambiguous candidates of the lane
+#pragma unroll
+  for (int c = 0; c < 2 * LANE_BINS; ++c) {
+    if (g[c] > P + K_RT_EPS) {
+      last = c;
+      last_gain = g[c];
+    } else if (g[c] > P) {
+      amb |= 1u << c;
+    }
+    P = fmax(P, g[c]);
+  }
+  const unsigned has = __ballot_sync(0xFFFFFFFFu, last >= 0);
+  const int owner = has ? 31 - __clz(has) : -1;
+  const int own_last = __shfl_sync(0xFFFFFFFFu, last, owner < 0 ? 0 : owner);
+  const double own_gain = __shfl_sync(0xFFFFFFFFu, last_gain, owner < 0 ? 0 : owner);
+  if (lane < owner) amb = 0;
+  if (lane == owner) amb &= ~((2u << last) - 1u);
+  int n = __popc(amb), before = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xFFFFFFFFu, before, o);
+    if (lane >= o) before += v;
+  }
+  const int total = __shfl_sync(0xFFFFFFFFu, before, 31);
+  before -= n;
+#pragma unroll
+  for (int c = 0; c < 2 * LANE_BINS; ++c)
+    if ((amb >> c) & 1u) {
+      if (before < AMB_MAX) {
+        rec->amb_gain[before] = g[c];
+        rec->amb_idx[before] = 2 * lane * N.e + c;
+      }
+      ++before;
+    }
+  if (lane == 0) {
+    rec->def_idx = owner < 0 ? -1 : 2 * owner * N.e + own_last;
+    rec->def_gain = own_gain;
+    rec->namb = total > AMB_MAX ? AMB_MAX + 1 : total;
+  }
+}
+
+// A node's split from the chosen candidate (found, with gain b); one warp.
+__device__ void write_split(const BState& S, size_t ni, const NodeSplit* best, bool found, double b) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  NodeSplit& o = S.split[ni];
+  if (lane == 0) {
+    found = found && b > K_RT_EPS;
+    o.loss_chg = found ? b : 0.0;
+    o.lg = best->lg;
+    o.lh = best->lh;
+    o.rg = best->rg;
+    o.rh = best->rh;
+    o.wl = best->wl;
+    o.wr = best->wr;
+    o.feature = best->feature;
+    o.bin = best->bin;
+    o.default_left = best->default_left;
+    o.is_cat = best->is_cat;
+    o.ncat = best->is_cat ? best->ncat : 0;
+    o.valid = found && b > S.gamma && best->lh >= S.reg.mcw && best->rh >= S.reg.mcw ? 1 : 0;
+  }
+  if (best->is_cat) {
+    for (int i = lane; i < MAX_CAT_BINS / 32; i += 32) o.cat_mask[i] = best->cat_mask[i];
+    for (int i = lane; i < best->ncat; i += 32) o.cat_order[i] = best->cat_order[i];
+  }
+}
+
+// Split search of a level in one launch, one warp per (frontier node, usable
+// pool feature) and then one block per node.
+//  1. Every warp materialises its feature's bins of a node whose histogram is
+//     the parent's minus the built sibling's (the subtraction trick, K5) and
+//     records the feature's best candidate (-inf when the node may not use
+//     the feature).
+//  2. The node's last block to finish applies consider's rule (g > best +
+//     1e-6, candidates in order): the first feature with the node's best gain
+//     holds the split when that gain is clear of every earlier feature's and
+//     of every earlier candidate of its own (by CLEAR, far above what up to
+//     576 records of at most 1e-6 each could add up to: it is then taken from
+//     any state the rule can be in, and nothing later exceeds it).
+//  3. Otherwise the rule is run in full: the features whose best gain is above
+//     every earlier one's (only these can hold records), their last certain
+//     record and the ambiguous ones after it (FeatRec), a warp per feature,
+//     then the last certain record over all features and a short sequential
+//     resolution over the ambiguous records after it.
+// Bound by latency: a chain of dependent loads, shuffles and f64 operations
+// per step. As three launches of 32-bin steps the phases took 35 us a level at
+// 100k x 30 and 60 us a lossguide step at 2M x 200 x 10 classes.
+__device__ __forceinline__ void k_eval_body(const BState& S, unsigned bx, int d) {
+  extern __shared__ double2 ev_sm[];
+  __shared__ double s_gains[SCAN_WARPS][64];
+  __shared__ uint16_t s_list[4096];  // pool positions of features whose best gain is a prefix maximum
+  __shared__ double s_wmax[SCAN_WARPS];
+  __shared__ int s_n, s_wcnt[SCAN_WARPS];
+  __shared__ bool s_last, s_decided;
+  __shared__ NodeSplit s_best;
   const int slot = bx, k = blockIdx.z;
   if (k >= S.K || slot >= S.lvl_count[k]) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pi = blockIdx.y * SCAN_WARPS + warp;
-  if (pi >= S.upool_len[k]) return;
-  const int f = (int)S.upool[(size_t)k * S.F + pi];
+  const int npool = S.upool_len[k];
+  const int nblocks = max(1, (npool + SCAN_WARPS - 1) / SCAN_WARPS);
+  if ((int)blockIdx.y >= nblocks) return;
+  const uint32_t* pool = S.upool + (size_t)k * S.F;
   const int nid = S.lvl_begin[k] + slot;
   const size_t ni = NI(S, k, nid);
   char* H = frontier_hist(S, d, k, slot);
-  if (d > 0 && !S.built[ni]) {
-    const char* P = parent_hist(S, d, k, ni);
-    const char* B = frontier_hist(S, d, k, slot ^ 1);
-    const int fs = (int)S.foff[f], nb = (int)S.foff[f + 1] - fs;
-    for (int i = lane; i <= nb; i += 32) {
-      const int e = i < nb ? fs + i : S.total_bins + f;  // bins, then the missing bin
-      if (S.fixed) {
-        longlong2 x = reinterpret_cast<const longlong2*>(P)[e], y = reinterpret_cast<const longlong2*>(B)[e];
-        reinterpret_cast<longlong2*>(H)[e] = make_longlong2(x.x - y.x, x.y - y.y);
-      } else {
-        double2 x = reinterpret_cast<const double2*>(P)[e], y = reinterpret_cast<const double2*>(B)[e];
-        reinterpret_cast<double2*>(H)[e] = make_double2(dsub(x.x, y.x), dsub(x.y, y.y));
+  double* M = S.mbuf + ((size_t)k * S.maxw + slot) * S.F;
+  FeatRec* R = S.frec + ((size_t)k * S.maxw + slot) * S.F;
+  double2* wsm = reinterpret_cast<double2*>(reinterpret_cast<char*>(ev_sm) + warp * eval_warp_bytes(S.cat_bins));
+  CatScratch csv{};
+  if (S.cat_cap > 0) csv = cat_scratch(reinterpret_cast<double*>(wsm), 0, S.cat_bins);
+  CatScratch* cs = S.cat_cap > 0 ? &csv : nullptr;
+  auto in_regs = [&](int f) { return !S.is_cat[f] && (int)(S.foff[f + 1] - S.foff[f]) <= NUM_BINS; };
+  const EvalNode E = eval_node(S, k, ni, d);
+  const int pi = blockIdx.y * SCAN_WARPS + warp;
+  if (pi < npool) {
+    const int f = (int)pool[pi];
+    const bool derive = d > 0 && !S.built[ni], wanted = in_mask(S.fmask + ni * S.FW, f);
+    const char* P = derive ? parent_hist(S, d, k, ni) : nullptr;
+    const char* B = derive ? frontier_hist(S, d, k, slot ^ 1) : nullptr;
+    double m = -INFINITY;
+    if (in_regs(f)) {
+      if (derive || wanted) {
+        NumScan N;
+        num_load(S, H, P, B, k, f, wsm, &N);
+        if (wanted) m = num_best(S, N, E, f, S.fbest + ((size_t)k * S.maxw + slot) * S.F + pi);
+      }
+    } else {
+      if (derive) {
+        const int fs = (int)S.foff[f], nb = (int)S.foff[f + 1] - fs;
+        for (int i = lane; i <= nb; i += 32) {
+          const int e = i < nb ? fs + i : S.total_bins + f;  // bins, then the missing bin
+          if (S.fixed) {
+            longlong2 x = reinterpret_cast<const longlong2*>(P)[e], y = reinterpret_cast<const longlong2*>(B)[e];
+            reinterpret_cast<longlong2*>(H)[e] = make_longlong2(x.x - y.x, x.y - y.y);
+          } else {
+            double2 x = reinterpret_cast<const double2*>(P)[e], y = reinterpret_cast<const double2*>(B)[e];
+            reinterpret_cast<double2*>(H)[e] = make_double2(dsub(x.x, y.x), dsub(x.y, y.y));
+          }
+        }
+        __syncwarp();
+      }
+      if (wanted) {
+        const Chosen c = scan_feature<SCAN_MAX>(S, H, k, f, E, 0.0, cs, nullptr, nullptr);
+        m = c.gain;
+        if (lane == 0)
+          S.fbest[((size_t)k * S.maxw + slot) * S.F + pi] =
+              FeatBest{0.0, 0.0, 0.0, 0.0, c.cand, c.before < dsub(m, CLEAR) ? 1 : 0, f, 0};
       }
     }
-    __syncwarp();
+    if (lane == 0) M[pi] = m;  // by pool position
   }
-  double m = -INFINITY;
-  if (in_mask(S.fmask + ni * S.FW, f)) {
-    const EvalNode E = eval_node(S, k, ni, d);
-    CatScratch csv{};
-  if (S.cat_cap > 0) csv = cat_scratch(ev_sm, warp, S.cat_bins);
-  CatScratch* cs = S.cat_cap > 0 ? &csv : nullptr;
-    m = scan_feature<SCAN_MAX>(S, H, k, f, E, 0.0, cs, nullptr, nullptr).gain;
+  // the node's last block goes on (its count is back at 0 for the next level)
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned* done = S.eval_done + (size_t)k * S.maxw + slot;
+    s_last = nblocks == 1 || atomicAdd(done, 1u) == (unsigned)nblocks - 1u;
+    if (s_last && nblocks > 1) *done = 0u;
+    s_n = 0;
   }
-  if (lane == 0) S.mbuf[((size_t)k * S.maxw + slot) * S.F + f] = m;
-}
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_scan(BState S, int d) { k_eval_scan_body(S, blockIdx.x, gridDim.x, d); }
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_scan_jobs(JobGrid J, int d) {
-  const int j = job_of(J, blockIdx.x);
-  k_eval_scan_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d);
-}
-
-// Phase 2a, one warp per (frontier node, usable pool feature): with Q = the
-// best gain of the node's earlier features (or 0), find this feature's last
-// certain record and its ambiguous records (FeatRec).
-__device__ __forceinline__ void k_eval_records_body(const BState& S, unsigned bx, unsigned gdx, int d) {
-  extern __shared__ double ev_sm[];
-  __shared__ double s_gains[SCAN_WARPS][64];
-  const int slot = bx, k = blockIdx.z;
-  if (k >= S.K || slot >= S.lvl_count[k]) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pi = blockIdx.y * SCAN_WARPS + warp;
-  if (pi >= S.upool_len[k]) return;
-  const int f = (int)S.upool[(size_t)k * S.F + pi];
-  const int nid = S.lvl_begin[k] + slot;
-  const size_t ni = NI(S, k, nid);
-  const size_t ri = ((size_t)k * S.maxw + slot) * S.F + f;
-  FeatRec* rec = S.frec + ri;
-  const double* M = S.mbuf + ((size_t)k * S.maxw + slot) * S.F;
-  if (!(M[f] > K_RT_EPS)) {  // no candidate can be taken from any state >= 0
-    if (lane == 0) {
-      rec->def_idx = -1;
-      rec->namb = 0;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // 2. the first feature with the best gain, and the best of the earlier ones
+  if (warp == 0) {
+    double top = -INFINITY;
+    int at = 0x7FFFFFFF;
+    for (int p = lane; p < npool; p += 32) {
+      const double g = __ldcg(M + p);
+      if (g > top) {
+        top = g;
+        at = p;
+      }
     }
-    return;
-  }
-  const uint32_t* fm = S.fmask + ni * S.FW;
-  double q = 0.0;  // max over the node's earlier features (only masked slots are current)
-  for (int j = lane; j < f; j += 32)
-    if (in_mask(fm, j)) q = fmax(q, M[j]);
-  q = warp_max(q);
-  // every record of this feature needs a gain above the running best, which
-  // starts at q: a feature whose best gain is not above q has none
-  if (!(M[f] > q)) {
-    if (lane == 0) {
-      rec->def_idx = -1;
-      rec->namb = 0;
+    const double all = warp_max(top);
+    int first = top == all ? at : 0x7FFFFFFF;
+    for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xFFFFFFFFu, first, o));
+    double q = 0.0;
+    for (int p = lane; p < min(first, npool); p += 32) q = fmax(q, __ldcg(M + p));
+    q = warp_max(q);
+    const bool none = !(all > K_RT_EPS);  // no candidate can be taken from any state >= 0
+    FeatBest fb{0.0, 0.0, 0.0, 0.0, 0, 1, -1, 0};
+    if (!none) {
+      const FeatBest* src = S.fbest + ((size_t)k * S.maxw + slot) * S.F + first;
+      const double2 a = __ldcg(reinterpret_cast<const double2*>(src)), c = __ldcg(reinterpret_cast<const double2*>(src) + 1);
+      const int4 i = __ldcg(reinterpret_cast<const int4*>(src) + 2);
+      fb = FeatBest{a.x, a.y, c.x, c.y, i.x, i.y, i.z, i.w};
     }
-    return;
+    const bool decided = none || (fb.clear && all > q + CLEAR);
+    const int f = fb.feature;
+    double wl = 0.0, wr = 0.0;
+    if (fb.sums && S.constrained)
+      cand_gain(S, E, S.mono ? S.mono[f] : 0, fb.lg, fb.lh, fb.rg, fb.rh, &wl, &wr);
+    if (lane == 0) {
+      s_decided = decided;
+      s_best.feature = fb.sums ? f : -1;
+      s_best.is_cat = 0;
+      s_best.ncat = 0;
+      s_best.default_left = fb.sums ? fb.idx & 1 : 1;
+      s_best.bin = fb.sums ? fb.idx >> 1 : 0;
+      s_best.lg = fb.lg;
+      s_best.lh = fb.lh;
+      s_best.rg = fb.rg;
+      s_best.rh = fb.rh;
+      s_best.wl = wl;
+      s_best.wr = wr;
+      if (d == 0) S.stats[ni] = make_double2(E.tg, E.th);
+    }
+    if (decided) {
+      if (f >= 0 && !fb.sums) {
+        __syncwarp();
+        scan_feature<SCAN_EXTRACT>(S, H, k, f, E, 0.0, cs, nullptr, &s_best, nullptr, fb.idx);
+      }
+      write_split(S, ni, &s_best, f >= 0, all);
+    }
   }
-  const EvalNode E = eval_node(S, k, ni, d);
-  CatScratch csv{};
-  if (S.cat_cap > 0) csv = cat_scratch(ev_sm, warp, S.cat_bins);
-  CatScratch* cs = S.cat_cap > 0 ? &csv : nullptr;
-  scan_feature<SCAN_RECORDS>(S, frontier_hist(S, d, k, slot), k, f, E, q, cs, s_gains[warp], nullptr, rec);
-}
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_records(BState S, int d) { k_eval_records_body(S, blockIdx.x, gridDim.x, d); }
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_records_jobs(JobGrid J, int d) {
-  const int j = job_of(J, blockIdx.x);
-  k_eval_records_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d);
-}
-
-// Phase 2b, one warp per frontier node: the winner of consider's sequential
-// rule is the last certain record over all features, followed by a short
-// sequential resolution over the ambiguous records after it.
-__device__ __forceinline__ void k_eval_pick_body(const BState& S, unsigned bx, unsigned gdx, int d) {
-  extern __shared__ double ev_sm[];
-  __shared__ NodeSplit s_best[SCAN_WARPS];
-  __shared__ double s_gains[SCAN_WARPS][64];
-  const int k = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (k >= S.K) return;
-  const int slot = bx * SCAN_WARPS + warp;
-  if (slot >= S.lvl_count[k]) return;
-  const int nid = S.lvl_begin[k] + slot;
-  const size_t ni = NI(S, k, nid);
-  const char* H = frontier_hist(S, d, k, slot);
-  const EvalNode E = eval_node(S, k, ni, d);
-  NodeSplit* best = &s_best[warp];
-  const double* M = S.mbuf + ((size_t)k * S.maxw + slot) * S.F;
-  const FeatRec* R = S.frec + ((size_t)k * S.maxw + slot) * S.F;
-  const uint32_t* fm = S.fmask + ni * S.FW;
-  CatScratch csv{};
-  if (S.cat_cap > 0) csv = cat_scratch(ev_sm, warp, S.cat_bins);
-  CatScratch* cs = S.cat_cap > 0 ? &csv : nullptr;
-  // last feature holding a certain record
-  int fstar = -1;
-  for (int j = lane; j < S.F; j += 32)
-    if (in_mask(fm, j) && M[j] > K_RT_EPS && R[j].def_idx >= 0) fstar = j;
-  for (int o = 16; o > 0; o >>= 1) fstar = max(fstar, __shfl_xor_sync(0xFFFFFFFFu, fstar, o));
+  __syncthreads();
+  if (s_decided) return;
+  // 3. strict prefix maxima of the features' best gains, from 0
+  double carry = 0.0;
+  for (int p0 = 0; p0 < npool; p0 += EVAL_THREADS) {
+    const int p = p0 + threadIdx.x;
+    const double g = p < npool ? __ldcg(M + p) : -INFINITY;
+    double incl = g;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl = fmax(incl, y);
+    }
+    if (lane == 31) s_wmax[warp] = incl;
+    __syncthreads();
+    double before = carry;
+    for (int w = 0; w < SCAN_WARPS; ++w) {
+      if (w < warp) before = fmax(before, s_wmax[w]);
+      carry = fmax(carry, s_wmax[w]);
+    }
+    const double up = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+    if (lane) before = fmax(before, up);
+    const unsigned rise = __ballot_sync(0xFFFFFFFFu, g > before);
+    if (lane == 0) s_wcnt[warp] = __popc(rise);
+    __syncthreads();
+    int at = s_n;
+    for (int w = 0; w < warp; ++w) at += s_wcnt[w];
+    if ((rise >> lane) & 1u) s_list[at + __popc(rise & ((1u << lane) - 1u))] = (uint16_t)p;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 0; w < SCAN_WARPS; ++w) s_n += s_wcnt[w];
+    __syncthreads();
+  }
+  const int n = s_n;
+  for (int i = warp; i < n; i += SCAN_WARPS) {
+    const int f = (int)pool[s_list[i]];
+    if (!(__ldcg(M + s_list[i]) > K_RT_EPS)) continue;  // no candidate can be taken from any state >= 0
+    const double q = i ? __ldcg(M + s_list[i - 1]) : 0.0;
+    if (in_regs(f)) {
+      NumScan N;
+      num_load(S, H, nullptr, nullptr, k, f, wsm, &N);
+      num_records(S, N, E, f, q, R + f);
+    } else {
+      scan_feature<SCAN_RECORDS>(S, H, k, f, E, q, cs, s_gains[warp], nullptr, R + f);
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  // the last feature holding a certain record, and what follows it
+  int istar = -1;
+  for (int i = lane; i < n; i += 32)
+    if (__ldcg(M + s_list[i]) > K_RT_EPS && R[pool[s_list[i]]].def_idx >= 0) istar = i;
+  for (int o = 16; o > 0; o >>= 1) istar = max(istar, __shfl_xor_sync(0xFFFFFFFFu, istar, o));
   double b = 0.0;
   int cf = -1, cidx = -1;
-  if (fstar >= 0) {
-    b = R[fstar].def_gain;
-    cf = fstar;
-    cidx = R[fstar].def_idx;
+  if (istar >= 0) {
+    cf = (int)pool[s_list[istar]];
+    b = R[cf].def_gain;
+    cidx = R[cf].def_idx;
   }
-  // ambiguous records after the winner, in candidate order: 32 features are
-  // tested at a time, and the (rare) features holding any are walked in order
-  for (int f0 = fstar < 0 ? 0 : fstar; f0 < S.F; f0 += 32) {
-    const int fl = f0 + lane;
-    const bool has = fl < S.F && in_mask(fm, fl) && M[fl] > K_RT_EPS && R[fl].namb > 0;
+  // 32 features are tested at a time, and the (rare) features holding
+  // ambiguous records are walked in order
+  for (int i0 = istar < 0 ? 0 : istar; i0 < n; i0 += 32) {
+    const int il = i0 + lane;
+    const bool has = il < n && __ldcg(M + s_list[il]) > K_RT_EPS && R[pool[s_list[il]]].namb > 0;
     unsigned hm = __ballot_sync(0xFFFFFFFFu, has);
     while (hm) {
-      const int f = f0 + __ffs(hm) - 1;
+      const int f = (int)pool[s_list[i0 + __ffs(hm) - 1]];
       hm &= hm - 1;
       const FeatRec& r = R[f];
       if (r.namb > AMB_MAX) {  // overflow: exact replay of this feature from b
-        Chosen c = scan_feature<SCAN_REPLAY>(S, H, k, f, E, b, cs, s_gains[warp], nullptr);
+        Chosen c = scan_feature<SCAN_REPLAY>(S, H, k, f, E, b, cs, s_gains[0], nullptr);
         if (c.cand >= 0) {
           b = c.gain;
           cf = f;
@@ -1154,46 +1535,38 @@ __device__ __forceinline__ void k_eval_pick_body(const BState& S, unsigned bx, u
         }
     }
   }
+  NodeSplit* best = &s_best;
   if (lane == 0) {
     best->feature = -1;
-    best->is_cat = 0;
-    best->ncat = 0;
     best->default_left = 1;
     best->bin = 0;
-    best->lg = best->lh = best->rg = best->rh = 0.0;
-    best->wl = best->wr = 0.0;
-    if (d == 0) S.stats[ni] = make_double2(E.tg, E.th);
+    best->lg = best->lh = best->rg = best->rh = best->wl = best->wr = 0.0;
   }
   __syncwarp();
-  if (cf >= 0) scan_feature<SCAN_EXTRACT>(S, H, k, cf, E, 0.0, cs, nullptr, best, nullptr, cidx);
-  __syncwarp();
-  NodeSplit& o = S.split[ni];
-  if (lane == 0) {
-    const bool found = cf >= 0 && b > K_RT_EPS;
-    const bool valid = found && b > S.gamma && best->lh >= S.reg.mcw && best->rh >= S.reg.mcw;
-    o.loss_chg = found ? b : 0.0;
-    o.lg = best->lg;
-    o.lh = best->lh;
-    o.rg = best->rg;
-    o.rh = best->rh;
-    o.wl = best->wl;
-    o.wr = best->wr;
-    o.feature = best->feature;
-    o.bin = best->bin;
-    o.default_left = best->default_left;
-    o.is_cat = best->is_cat;
-    o.ncat = best->is_cat ? best->ncat : 0;
-    o.valid = valid ? 1 : 0;
+  if (cf >= 0 && in_regs(cf)) {  // the chosen candidate's statistics, from the scan's own sums
+    NumScan N;
+    num_load(S, H, nullptr, nullptr, k, cf, wsm, &N);
+    if (lane == 0) {
+      double2 l, r;
+      num_sides(N, E, cidx, &l, &r);
+      best->feature = cf;
+      best->bin = cidx >> 1;
+      best->default_left = cidx & 1;
+      best->lg = l.x;
+      best->lh = l.y;
+      best->rg = r.x;
+      best->rh = r.y;
+      cand_gain(S, E, S.mono ? S.mono[cf] : 0, l.x, l.y, r.x, r.y, &best->wl, &best->wr);
+    }
+  } else if (cf >= 0) {
+    scan_feature<SCAN_EXTRACT>(S, H, k, cf, E, 0.0, cs, nullptr, best, nullptr, cidx);
   }
-  if (cf >= 0 && best->is_cat) {
-    for (int i = lane; i < MAX_CAT_BINS / 32; i += 32) o.cat_mask[i] = best->cat_mask[i];
-    for (int i = lane; i < best->ncat; i += 32) o.cat_order[i] = best->cat_order[i];
-  }
+  write_split(S, ni, best, cf >= 0, b);
 }
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_pick(BState S, int d) { k_eval_pick_body(S, blockIdx.x, gridDim.x, d); }
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval_pick_jobs(JobGrid J, int d) {
+__global__ void __launch_bounds__(EVAL_THREADS) k_eval(BState S, int d) { k_eval_body(S, blockIdx.x, d); }
+__global__ void __launch_bounds__(EVAL_THREADS) k_eval_jobs(JobGrid J, int d) {
   const int j = job_of(J, blockIdx.x);
-  k_eval_pick_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d);
+  k_eval_body(J.states[j], blockIdx.x - J.xoff[j], d);
 }
 
 __device__ sb_node make_leaf(float value, float sum_hess) {  // Node::leaf, regtree.rs:51-65
@@ -1888,6 +2261,8 @@ struct sb_booster {
   sb::DBuf<int> d_pool_len, d_upool_len;
   sb::DBuf<double> d_mbuf;
   sb::DBuf<sb::FeatRec> d_frec;
+  sb::DBuf<sb::FeatBest> d_fbest;
+  sb::DBuf<unsigned> d_eval_done;
   sb::DBuf<uint32_t> d_samp;
   sb::DBuf<sb_node> d_out_nodes;
   sb::DBuf<uint32_t> d_out_cats;
@@ -2202,6 +2577,8 @@ int booster_init(sb_booster* b, sb_ctx* ctx, const sb_ghist* g, const sb_train_p
   SB_TRY(b->d_pool_mask.alloc_zero(ctx, (size_t)K * FW));
   SB_TRY(b->d_mbuf.alloc_zero(ctx, (size_t)K * b->maxw * F));
   SB_TRY(b->d_frec.alloc_zero(ctx, (size_t)K * b->maxw * F));
+  SB_TRY(b->d_fbest.alloc_zero(ctx, (size_t)K * b->maxw * F));
+  SB_TRY(b->d_eval_done.alloc_zero(ctx, (size_t)K * b->maxw));
   {
     std::vector<uint32_t> usable(FW, 0u);
     for (int f = 0; f < F; ++f)
@@ -2324,6 +2701,8 @@ int booster_init(sb_booster* b, sb_ctx* ctx, const sb_ghist* g, const sb_train_p
   S.usable = b->d_usable.p;
   S.mbuf = b->d_mbuf.p;
   S.frec = b->d_frec.p;
+  S.fbest = b->d_fbest.p;
+  S.eval_done = b->d_eval_done.p;
   S.samp_scratch = b->d_samp.p;
   S.row_leaf = nullptr;
   SB_TRY(booster_alloc_trees(b, K * 16));
@@ -2331,7 +2710,7 @@ int booster_init(sb_booster* b, sb_ctx* ctx, const sb_ghist* g, const sb_train_p
 }
 
 size_t eval_smem(const sb_booster* b) {
-  return b->S.cat_cap ? (EVAL_THREADS / 32) * cat_scratch_bytes(b->S.cat_bins) : 0;
+  return SCAN_WARPS * eval_warp_bytes(b->S.cat_bins);
 }
 
 // The launches of one boosting round on the context stream (also recorded into
@@ -2408,11 +2787,7 @@ int booster_round_body(sb_booster* b, int apply_delta) {
     const unsigned fy = (unsigned)((b->g->F + SCAN_WARPS - 1) / SCAN_WARPS);
     const size_t heap_smem = (size_t)b->maxn * sizeof(HeapEnt);
     auto eval = [&](int d, unsigned width) -> int {
-      dim3 sg(width, fy, (unsigned)b->K);
-      SB_LAUNCH(ctx, k_eval_scan, sg, EVAL_THREADS, esm, S, d);
-      SB_LAUNCH(ctx, k_eval_records, sg, EVAL_THREADS, esm, S, d);
-      dim3 pg(1, (unsigned)b->K);
-      SB_LAUNCH(ctx, k_eval_pick, pg, EVAL_THREADS, esm, S, d);
+      SB_LAUNCH(ctx, k_eval, dim3(width, fy, (unsigned)b->K), EVAL_THREADS, esm, S, d);
       return SB_OK;
     };
     SB_TRY(eval(0, 1));  // the root
@@ -2435,10 +2810,7 @@ int booster_round_body(sb_booster* b, int apply_delta) {
   for (int d = 0; d < b->D && !b->lossguide; ++d) {
     const unsigned width = (unsigned)std::min(1 << d, b->maxw);
     dim3 sg(width, (unsigned)((b->g->F + SCAN_WARPS - 1) / SCAN_WARPS), (unsigned)b->K);
-    SB_LAUNCH(ctx, k_eval_scan, sg, EVAL_THREADS, esm, S, d);
-    SB_LAUNCH(ctx, k_eval_records, sg, EVAL_THREADS, esm, S, d);
-    dim3 pg((width + SCAN_WARPS - 1) / SCAN_WARPS, (unsigned)b->K);
-    SB_LAUNCH(ctx, k_eval_pick, pg, EVAL_THREADS, esm, S, d);
+    SB_LAUNCH(ctx, k_eval, sg, EVAL_THREADS, esm, S, d);
     // 1024 threads: the threads also write the level's partition tiles (about
     // n / PART_TILE at the root), one binary search each
     SB_LAUNCH(ctx, k_assign, assign_blocks(b, 1024), 1024, 0, S, d, 1);
@@ -2536,9 +2908,7 @@ int booster_collect_timing(sb_booster* b) {
 
 int booster_set_eval_smem(sb_booster* b) {
   int esm = (int)eval_smem(b);
-  SB_TRY(raise_smem_limit((const void*)k_eval_scan, (size_t)esm));
-  SB_TRY(raise_smem_limit((const void*)k_eval_pick, (size_t)esm));
-  SB_TRY(raise_smem_limit((const void*)k_eval_records, (size_t)esm));
+  SB_TRY(raise_smem_limit((const void*)k_eval, (size_t)esm));
   if (b->lossguide) {
     const size_t heap_smem = (size_t)b->maxn * sizeof(HeapEnt);
     SB_REQUIRE(heap_smem <= b->ctx->smem_optin, SB_ERR_UNSUPPORTED, "lossguide queue of %d nodes exceeds shared memory",
@@ -2669,9 +3039,7 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
     maxK = std::max(maxK, b->K);
     esm = std::max(esm, eval_smem(b));
   }
-  SB_TRY(raise_smem_limit((const void*)k_eval_scan_jobs, esm));
-  SB_TRY(raise_smem_limit((const void*)k_eval_records_jobs, esm));
-  SB_TRY(raise_smem_limit((const void*)k_eval_pick_jobs, esm));
+  SB_TRY(raise_smem_limit((const void*)k_eval_jobs, esm));
   // the histogram launches' per-job descriptions
   std::vector<HistLaunch> Ls(nb);
   for (int j = 0; j < nb; ++j) {
@@ -2722,7 +3090,7 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
   const Step s_quant = step([&](int j) { return fixed ? gblocks(j) : 0; });
   const Step s_hist0 = step([&](int j) { return hp.hist_grid[j]; });
   const Step s_zero0 = step([&](int j) { return hp.zero_grid[j]; });
-  std::vector<Step> s_scan(maxD), s_pick(maxD), s_assign(maxD), s_part(maxD), s_plan(maxD), s_hist(maxD),
+  std::vector<Step> s_scan(maxD), s_assign(maxD), s_part(maxD), s_plan(maxD), s_hist(maxD),
       s_zero(maxD);
   std::vector<unsigned> fy(maxD, 1);
   std::vector<int> items(maxD, 0);
@@ -2731,7 +3099,6 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
     auto act = [&](int j) { return d < bs[j]->D; };
     auto build = [&](int j) { return d + 1 < bs[j]->D; };
     s_scan[d] = step([&](int j) { return act(j) ? width(j) : 0u; });
-    s_pick[d] = step([&](int j) { return act(j) ? (width(j) + SCAN_WARPS - 1) / SCAN_WARPS : 0u; });
     s_assign[d] = step([&](int j) { return act(j) ? assign_blocks(bs[j], 1024) : 0u; });
     s_part[d] = step([&](int j) {
       return act(j) ? part_blocks(ctx, bs[j]->n, bs[j]->K, (size_t)bs[j]->K * width(j)) : 0u;
@@ -2762,10 +3129,7 @@ int boosters_train_batched(sb_ctx* ctx, sb_booster* const* bs, int nb, int round
     for (int d = 0; d < maxD; ++d) {
       if (s_scan[d].blocks == 0) break;
       const dim3 sg(s_scan[d].blocks, fy[d], (unsigned)maxK);
-      SB_LAUNCH(ctx, k_eval_scan_jobs, sg, EVAL_THREADS, esm, J(d_states.p, s_scan[d]), d);
-      SB_LAUNCH(ctx, k_eval_records_jobs, sg, EVAL_THREADS, esm, J(d_states.p, s_scan[d]), d);
-      SB_LAUNCH(ctx, k_eval_pick_jobs, dim3(s_pick[d].blocks, (unsigned)maxK), EVAL_THREADS, esm,
-                J(d_states.p, s_pick[d]), d);
+      SB_LAUNCH(ctx, k_eval_jobs, sg, EVAL_THREADS, esm, J(d_states.p, s_scan[d]), d);
       SB_LAUNCH(ctx, k_assign_jobs, s_assign[d].blocks, 1024, 0, J(d_states.p, s_assign[d]), d, 1);
       SB_LAUNCH(ctx, k_partition_jobs, s_part[d].blocks, PART_THREADS, 0, J(d_states.p, s_part[d]), d);
       if (s_plan[d].blocks) {
