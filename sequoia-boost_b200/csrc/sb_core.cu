@@ -154,17 +154,22 @@ int sb_ctx_create(int device, sb_ctx** out) {
     return SB_ERR_NO_DEVICE;
   }
   SB_REQUIRE(device >= 0 && device < count, SB_ERR_INVALID_ARG, "device %d out of range", device);
-  cudaDeviceProp prop;
-  SB_CUDA(cudaGetDeviceProperties(&prop, device));
-  SB_REQUIRE(prop.major == 10 && prop.minor == 0, SB_ERR_NO_DEVICE,
-             "device %d is sm_%d%d; this library is built for sm_100a (B200) only", device,
-             prop.major, prop.minor);
+  // single attributes: cudaGetDeviceProperties takes milliseconds a call, and
+  // sb_train_many opens a context per stream
+  int major = 0, minor = 0, sms = 0, optin = 0, per_sm = 0;
+  SB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  SB_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  SB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  SB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  SB_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+  SB_REQUIRE(major == 10 && minor == 0, SB_ERR_NO_DEVICE,
+             "device %d is sm_%d%d; this library is built for sm_100a (B200) only", device, major, minor);
   SB_CUDA(cudaSetDevice(device));
   sb_ctx* c = new sb_ctx;
   c->device = device;
-  c->num_sms = prop.multiProcessorCount;
-  c->smem_optin = prop.sharedMemPerBlockOptin;
-  c->smem_per_sm = prop.sharedMemPerMultiprocessor;
+  c->num_sms = sms;
+  c->smem_optin = (size_t)optin;
+  c->smem_per_sm = (size_t)per_sm;
   cudaError_t se = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (se != cudaSuccess) {
     delete c;

@@ -2333,7 +2333,47 @@ namespace {
 
 // Objective::base_margin / prob_to_margin with TrainingParams::base_score
 // (learner/train.rs:203-210) from host labels and weights.
-float base_margin_of(const sb_train_params* p, const float* labels, const float* weights, size_t n, int K) {
+// Sum, sum of magnitudes and count of non-integers of n labels, into out[3].
+__global__ void __launch_bounds__(256) k_label_stats(const float* __restrict__ y, size_t n, double* __restrict__ out) {
+  double v[3] = {0.0, 0.0, 0.0};
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const float x = y[i];
+    v[0] += (double)x;
+    v[1] += fabs((double)x);
+    v[2] += x == rintf(x) && fabsf(x) < INFINITY ? 0.0 : 1.0;
+  }
+  for (int j = 0; j < 3; ++j) {
+    v[j] = warp_sum(v[j]);
+    if ((threadIdx.x & 31) == 0) atomicAdd(out + j, v[j]);
+  }
+}
+__global__ void k_fill(float* __restrict__ p, size_t n, float v) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
+}
+
+// The labels' sum where every partial sum is an integer below 2^53: exact in
+// f64, so the device's sum in any order is the sequential one (class labels,
+// counts). A long vector's sequential additions take a nanosecond each on the
+// host (10M labels 10 ms, this 0.05 ms). *exact = false otherwise.
+constexpr size_t LABEL_SUM_MIN = 65536;
+int label_sum(sb_ctx* ctx, const float* d_labels, size_t n, double* sum, bool* exact) {
+  *exact = false;
+  if (n < LABEL_SUM_MIN) return SB_OK;
+  DBuf<double> d;
+  SB_TRY(d.alloc_zero(ctx, 3));
+  const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 8);
+  SB_LAUNCH(ctx, k_label_stats, blocks, 256, 0, d_labels, n, d.p);
+  double h[3];
+  SB_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  SB_CUDA(cudaStreamSynchronize(ctx->stream));
+  *exact = h[2] == 0.0 && h[1] < 9007199254740992.0;
+  *sum = h[0];
+  return SB_OK;
+}
+
+// known_sum: the labels' sum where it is known already, or null.
+float base_margin_of(const sb_train_params* p, const float* labels, const float* weights, size_t n, int K,
+                     const double* known_sum = nullptr) {
   float base;
   if (K > 1) base = 0.0f;
   else if (p->has_base_score) {
@@ -2355,7 +2395,9 @@ float base_margin_of(const sb_train_params* p, const float* labels, const float*
       mean = den > 0.0 ? num / den : 0.0;
     } else {
       double sum = 0.0;
-      for (size_t i = 0; i < n; ++i) sum += (double)labels[i];
+      if (known_sum) sum = *known_sum;
+      else
+        for (size_t i = 0; i < n; ++i) sum += (double)labels[i];
       mean = sum / (double)n;
     }
     if (p->objective == SB_OBJ_LOGISTIC) {
@@ -3428,26 +3470,29 @@ int sb_booster_create(sb_ctx* ctx, const sb_ghist* g, const sb_train_params* p, 
     delete b;
     return s;
   }
-  const float base = base_margin_of(p, labels, weights, n, K);
-  b->base_score = base;
-  std::vector<float> m(n * K, base);  // init_margin, train.rs:496-511
-  if (base_margin) std::memcpy(m.data(), base_margin, n * K * sizeof(float));
   cudaStream_t st = ctx->stream;
-  if ((s = b->d_labels.alloc(ctx, n)) != SB_OK) { delete b; return s; }
-  cudaMemcpyAsync(b->d_labels.p, labels, n * 4, cudaMemcpyHostToDevice, st);
+  std::unique_ptr<sb_booster> own(b);
+  SB_TRY(b->d_labels.alloc(ctx, n));
+  SB_CUDA(cudaMemcpyAsync(b->d_labels.p, labels, n * 4, cudaMemcpyHostToDevice, st));
   if (weights) {
-    if ((s = b->d_weights.alloc(ctx, n)) != SB_OK) { delete b; return s; }
-    cudaMemcpyAsync(b->d_weights.p, weights, n * 4, cudaMemcpyHostToDevice, st);
+    SB_TRY(b->d_weights.alloc(ctx, n));
+    SB_CUDA(cudaMemcpyAsync(b->d_weights.p, weights, n * 4, cudaMemcpyHostToDevice, st));
   }
-  cudaMemcpyAsync(b->d_margin.p, m.data(), n * K * 4, cudaMemcpyHostToDevice, st);
+  double sum = 0.0;
+  bool exact = false;
+  if (K == 1 && !p->has_base_score && !weights) SB_TRY(label_sum(ctx, b->d_labels.p, n, &sum, &exact));
+  const float base = base_margin_of(p, labels, weights, n, K, exact ? &sum : nullptr);
+  b->base_score = base;
+  if (base_margin) {  // init_margin, train.rs:496-511
+    SB_CUDA(cudaMemcpyAsync(b->d_margin.p, base_margin, n * K * 4, cudaMemcpyHostToDevice, st));
+  } else {
+    const unsigned blocks = (unsigned)std::min<size_t>((n * K + 255) / 256, (size_t)ctx->num_sms * 16);
+    SB_LAUNCH(ctx, k_fill, blocks, 256, 0, b->d_margin.p, n * K, base);
+  }
   b->S.labels = b->d_labels.p;
   b->S.weights = b->d_weights.p;
-  cudaError_t e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    delete b;
-    return sb::cuda_status(e, "booster upload", __FILE__, __LINE__);
-  }
-  *out = b;
+  SB_CUDA(cudaStreamSynchronize(st));  // the caller's buffers are free on return
+  *out = own.release();
   return SB_OK;
 }
 
