@@ -317,6 +317,8 @@ struct PathEl {
 
 struct DevEnsemble {
   DBuf<int4> nodes;          // packed predict nodes
+  bool compact = false;      // every tree has the 8-byte form (cnodes)
+  DBuf<uint2> cnodes;
   DBuf<int> cat_end;         // per node: end of its category list
   DBuf<int64_t> tree_off;    // node offset per tree
   DBuf<uint32_t> cats;
@@ -378,7 +380,8 @@ int shap_prepare(sb_model* m);
 // per-row base margins d_base_margin ([n][K] when bm_kind == 1, [n] when 2),
 // plus the weighted leaf values of the first ntree_limit trees (0: all).
 int predict_margin_device(sb_model* m, const float* d_X, size_t n, size_t F, float missing,
-                          const float* d_base_margin, int bm_kind, size_t ntree_limit, float* d_out);
+                          const float* d_base_margin, int bm_kind, size_t ntree_limit, float* d_out,
+                          int transform_objective = -1);  // >= 0: a single output goes through pred_transform
 int predict_contribs_device(sb_model* m, const float* d_X, size_t n, size_t F, float missing, float* d_out);
 int predict_interactions_device(sb_model* m, const float* d_X, size_t n, size_t F, float missing,
                                 float* d_out);
