@@ -408,7 +408,9 @@ __device__ __forceinline__ void k_gradient_body(const BState& S, unsigned bx, un
   __syncthreads();
   if (S.fixed && tid < 2 * K && tid < 32 && s_max[tid]) atomicMax(&S.maxabs[tid], s_max[tid]);
 }
-__global__ void __launch_bounds__(256) k_gradient(BState S) { k_gradient_body(S, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(256) k_gradient(BState S) {
+  k_gradient_body(S, blockIdx.x, gridDim.x);
+}
 __global__ void __launch_bounds__(256) k_gradient_jobs(JobGrid J) {
   const int j = job_of(J, blockIdx.x);
   k_gradient_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j]);
@@ -441,7 +443,9 @@ __device__ __forceinline__ void k_route_rest_body(const BState& S, unsigned bx, 
     if (S.row_leaf) S.row_leaf[r] = -1;
   }
 }
-__global__ void k_route_rest(BState S) { k_route_rest_body(S, blockIdx.x, gridDim.x); }
+__global__ void k_route_rest(BState S) {
+  k_route_rest_body(S, blockIdx.x, gridDim.x);
+}
 __global__ void k_route_rest_jobs(JobGrid J) {
   const int j = job_of(J, blockIdx.x);
   k_route_rest_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j]);
@@ -607,7 +611,9 @@ __device__ __forceinline__ void k_round_prep_body(const BState& S, unsigned bx, 
     node_feature_mask(S, k, 0, tkey, S.fmask + NI(S, k, 0) * S.FW, nullptr, true,
                       S.samp_scratch ? S.samp_scratch + (size_t)k * S.F : nullptr);
 }
-__global__ void __launch_bounds__(PREP_THREADS) k_round_prep(BState S) { k_round_prep_body(S, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(PREP_THREADS) k_round_prep(BState S) {
+  k_round_prep_body(S, blockIdx.x, gridDim.x);
+}
 __global__ void __launch_bounds__(PREP_THREADS) k_round_prep_jobs(JobGrid J) {
   const int j = job_of(J, blockIdx.x);
   k_round_prep_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j]);
@@ -642,7 +648,9 @@ __device__ __forceinline__ void k_quantize_body(const BState& S, unsigned bx, un
   __syncthreads();
   if (threadIdx.x < 2 && s_e[threadIdx.x]) atomicMax((unsigned int*)&S.qerr[0] + threadIdx.x, s_e[threadIdx.x]);
 }
-__global__ void k_quantize(BState S) { k_quantize_body(S, blockIdx.x, gridDim.x); }
+__global__ void k_quantize(BState S) {
+  k_quantize_body(S, blockIdx.x, gridDim.x);
+}
 __global__ void k_quantize_jobs(JobGrid J) {
   const int j = job_of(J, blockIdx.x);
   k_quantize_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j]);
@@ -1563,7 +1571,9 @@ __device__ __forceinline__ void k_eval_body(const BState& S, unsigned bx, int d)
   }
   write_split(S, ni, best, cf >= 0, b);
 }
-__global__ void __launch_bounds__(EVAL_THREADS) k_eval(BState S, int d) { k_eval_body(S, blockIdx.x, d); }
+__global__ void __launch_bounds__(EVAL_THREADS) k_eval(BState S, int d) {
+  k_eval_body(S, blockIdx.x, d);
+}
 __global__ void __launch_bounds__(EVAL_THREADS) k_eval_jobs(JobGrid J, int d) {
   const int j = job_of(J, blockIdx.x);
   k_eval_body(J.states[j], blockIdx.x - J.xoff[j], d);
@@ -1588,10 +1598,14 @@ __device__ sb_node make_leaf(float value, float sum_hess) {  // Node::leaf, regt
 
 // Expand the frontier of level d: child ids in the reference's order
 // (left = num_nodes + 2 * rank among split nodes), child state, final leaf
-// values, and the level's partition tiles.
+// values, and the level's partition tiles. Bound by latency: a block's chain
+// of dependent loads and barriers. So a node's state and what its split
+// feature leads to are requested before the one scan that ranks the splits,
+// their categories and their tiles together (three scans and a reservation
+// before them: 8 us a level of up to 32 nodes, now 6).
 __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsigned gdx, int d, int write_tiles) {
-  __shared__ int sm_i[33];
-  __shared__ int s_tile_carry;
+  __shared__ unsigned long long sm_u[33];
+  __shared__ int s_tile0;
   __shared__ int s_toff[1024], s_nid[1024];
   __shared__ uint2 s_seg[1024];
   const unsigned long long round = *S.round;
@@ -1599,45 +1613,52 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
   const bool last = !S.lossguide && (d + 1 == S.max_depth);
   for (int k = bx; k < S.K; k += gdx) {  // one class tree per block
     const int begin = S.lvl_begin[k], cnt = S.lvl_count[k], nn0 = S.num_nodes[k];
-    if (write_tiles) {  // reserve the tree's partition tiles (their order in the list is free)
-      int mine = 0;
-      for (int q = tid; q < cnt; q += blockDim.x) {
-        const uint2 sg = S.seg[NI(S, k, begin + q)];
-        mine += (int)((sg.y - sg.x + PART_TILE - 1) / PART_TILE);
-      }
-      int all;
-      block_scan_excl<int>(mine, &all, sm_i);
-      if (tid == 0) s_tile_carry = all ? atomicAdd(S.ptile_count, all) : 0;
-      __syncthreads();
-    }
+    int carry_v = 0, carry_c = S.cat_count[k];
     const size_t t = (size_t)round * S.K + k;
     sb_node* out = S.out_nodes + t * S.maxn;
     uint32_t* ocats = S.out_cats ? S.out_cats + t * S.cat_cap : nullptr;
     const uint64_t tkey = sb_tree_key(S.seed, round + S.round_base, (uint64_t)(k + S.k_base));
-    int carry_v = 0, carry_c = S.cat_count[k];
     for (int c0 = 0; c0 < cnt; c0 += blockDim.x) {
       const int slot = c0 + tid;
       const bool act = slot < cnt;
       const int nid = begin + slot;
       const size_t ni = act ? NI(S, k, nid) : 0;
       const NodeSplit* sp = act ? &S.split[ni] : nullptr;
-      const int v = (act && sp->valid) ? 1 : 0;
-      const int nc = (v && sp->is_cat) ? sp->ncat : 0;
-      int tot_v, tot_c;
-      const int rank = carry_v + block_scan_excl<int>(v, &tot_v, sm_i);
-      const int coff = carry_c + block_scan_excl<int>(nc, &tot_c, sm_i);
-      int tiles = 0;
+      int v = 0, nc = 0, tiles = 0, f = 0, dr = 0;
+      bool is_cat = false, pall = true, fall = true;
+      uint2 sg = make_uint2(0u, 0u);
+      double2 st = make_double2(0.0, 0.0), bd = st;
+      float cond = 0.0f;
       if (act) {
-        const double2 st = S.stats[ni];
-        const double2 bd = S.bounds[ni];
-        if (d == 0) out[0] = make_leaf(0.0f, (float)st.y);  // RegTree::with_root
-        const uint2 sg = S.seg[ni];
+        sg = S.seg[ni];
+        st = S.stats[ni];
+        bd = S.bounds[ni];
+        pall = S.allowed_all[ni];
+        v = sp->valid ? 1 : 0;
+        is_cat = sp->is_cat != 0;
+        nc = v && is_cat ? sp->ncat : 0;
         tiles = (int)((sg.y - sg.x + PART_TILE - 1) / PART_TILE);
+        if (v) {
+          f = sp->feature;
+          dr = S.mono ? S.mono[f] : 0;
+          fall = !S.has_inter || !S.in_group[f];
+          if (!is_cat) cond = S.cuts[S.foff[f] + sp->bin];
+        }
+      }
+      // splits, categories and tiles before the node: 11, 27 and 26 bits
+      unsigned long long tot;
+      const unsigned long long mine = (unsigned long long)v | (unsigned long long)nc << 11 | (unsigned long long)tiles << 38;
+      const unsigned long long at = block_scan_excl<unsigned long long>(mine, &tot, sm_u);
+      const int tot_v = (int)(tot & 0x7FFu), tot_c = (int)((tot >> 11) & 0x7FFFFFFu), tot_t = (int)(tot >> 38);
+      const int rank = carry_v + (int)(at & 0x7FFu), coff = carry_c + (int)((at >> 11) & 0x7FFFFFFu);
+      const int toff = (int)(at >> 38);
+      // the trees' tiles come in any order; the reservation is back by the time they are written
+      if (write_tiles && tid == 0) s_tile0 = tot_t ? atomicAdd(S.ptile_count, tot_t) : 0;
+      if (act) {
+        if (d == 0) out[0] = make_leaf(0.0f, (float)st.y);  // RegTree::with_root
         S.fill[ni] = Fill{0u, 0u};
         if (v) {
           const int left = nn0 + 2 * rank, right = left + 1;
-          const int f = sp->feature;
-          const int dr = S.mono ? S.mono[f] : 0;
           double2 lb = bd, rb = bd;  // child_bounds, constraints.rs:94-124
           if (dr != 0) {
             double mid = dmul(0.5, dadd(sp->wl, sp->wr));
@@ -1650,7 +1671,7 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
           pn.left = left;
           pn.right = right;
           pn.split_gain = (float)sp->loss_chg;
-          if (sp->is_cat) {
+          if (is_cat) {
             pn.is_categorical = 1;
             pn.cat_begin = (uint32_t)coff;
             pn.cat_end = (uint32_t)(coff + sp->ncat);
@@ -1658,16 +1679,14 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
             for (int c = 0; c < sp->ncat; ++c)
               if (ocats && coff + c < S.cat_cap) ocats[coff + c] = f32_as_u32(S.cuts[fs + sp->cat_order[c]]);
           } else {
-            pn.split_cond = S.cuts[S.foff[f] + sp->bin];
+            pn.split_cond = cond;
           }
           out[left] = make_leaf((float)sp->wl, (float)sp->lh);
           out[right] = make_leaf((float)sp->wr, (float)sp->rh);
           // interaction constraints (intersect_allowed, hist.rs:736-747)
           const size_t li = NI(S, k, left), ri = NI(S, k, right);
-          const bool pall = S.allowed_all[ni];
-          const bool fall = !S.has_inter || !S.in_group[f];
           const bool call = pall && fall;
-          for (int w = 0; w < S.FW; ++w) {
+          for (int w = 0; w < S.FW && !call; ++w) {  // read only where not all are allowed
             uint32_t a = pall ? 0xFFFFFFFFu : S.allowed[ni * S.FW + w];
             uint32_t b = fall ? 0xFFFFFFFFu : S.iset[(size_t)f * S.FW + w];
             uint32_t x = a & b;
@@ -1708,12 +1727,10 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
       }
       // partition tiles of this chunk's frontier nodes: one thread per tile,
       // its node found by a binary search over the chunk's tile offsets
-      int tot_t;
-      const int toff = block_scan_excl<int>(tiles, &tot_t, sm_i);
       if (write_tiles) {
         s_toff[tid] = toff + tiles;  // inclusive end
         if (act) {
-          s_seg[tid] = S.seg[ni];
+          s_seg[tid] = sg;
           s_nid[tid] = nid;
         }
         __syncthreads();
@@ -1727,15 +1744,13 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
           const int qi = q - (s_toff[lo] - (int)((s_seg[lo].y - s_seg[lo].x + PART_TILE - 1) / PART_TILE));
           const unsigned b = s_seg[lo].x + (unsigned)qi * PART_TILE;
           const unsigned e = min(s_seg[lo].y, b + PART_TILE);
-          const int slot_t = s_tile_carry + q;
+          const int slot_t = s_tile0 + q;
           if (slot_t < S.ptile_cap) S.ptiles[slot_t] = make_int4(k, s_nid[lo], (int)b, (int)e);
         }
+        __syncthreads();
       }
-      __syncthreads();
-      if (tid == 0) s_tile_carry += tot_t;
       carry_v += tot_v;
       carry_c += tot_c;
-      __syncthreads();
     }
     __syncthreads();
     if (tid == 0) {
@@ -1749,7 +1764,9 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(1024) k_assign(BState S, int d, int write_tiles) { k_assign_body(S, blockIdx.x, gridDim.x, d, write_tiles); }
+__global__ void __launch_bounds__(1024) k_assign(BState S, int d, int write_tiles) {
+  k_assign_body(S, blockIdx.x, gridDim.x, d, write_tiles);
+}
 __global__ void __launch_bounds__(1024) k_assign_jobs(JobGrid J, int d, int write_tiles) {
   const int j = job_of(J, blockIdx.x);
   k_assign_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d, write_tiles);
@@ -1879,7 +1896,9 @@ __device__ __forceinline__ void k_partition_body(const BState& S, unsigned bx, u
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(PART_THREADS, 4) k_partition(BState S, int d) { k_partition_body(S, blockIdx.x, gridDim.x, d); }
+__global__ void __launch_bounds__(PART_THREADS, 4) k_partition(BState S, int d) {
+  k_partition_body(S, blockIdx.x, gridDim.x, d);
+}
 __global__ void __launch_bounds__(PART_THREADS, 4) k_partition_jobs(JobGrid J, int d) {
   const int j = job_of(J, blockIdx.x);
   k_partition_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d);
@@ -1980,7 +1999,9 @@ __device__ __forceinline__ void k_plan_body(const BState& S, unsigned bx, unsign
     *S.ptile_count = 0;  // the partition has consumed this level's tiles
   }
 }
-__global__ void __launch_bounds__(1024) k_plan(BState S, int d) { k_plan_body(S, blockIdx.x, gridDim.x, d); }
+__global__ void __launch_bounds__(1024) k_plan(BState S, int d) {
+  k_plan_body(S, blockIdx.x, gridDim.x, d);
+}
 __global__ void __launch_bounds__(1024) k_plan_jobs(JobGrid J, int d) {
   const int j = job_of(J, blockIdx.x);
   k_plan_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j], d);
@@ -2180,7 +2201,9 @@ __device__ __forceinline__ void k_round_end_body(const BState& S, unsigned bx, u
       for (int i = 0; i < 2 * S.K; ++i) S.maxabs[i] = 0u;
   }
 }
-__global__ void k_round_end(BState S) { k_round_end_body(S, blockIdx.x, gridDim.x); }
+__global__ void k_round_end(BState S) {
+  k_round_end_body(S, blockIdx.x, gridDim.x);
+}
 __global__ void k_round_end_jobs(JobGrid J) {
   const int j = job_of(J, blockIdx.x);
   k_round_end_body(J.states[j], blockIdx.x - J.xoff[j], J.xoff[j + 1] - J.xoff[j]);
