@@ -444,6 +444,7 @@ __device__ __forceinline__ void k_route_rest_body(const BState& S, unsigned bx, 
   }
 }
 __global__ void k_route_rest(BState S) {
+  follow_launch();
   k_route_rest_body(S, blockIdx.x, gridDim.x);
 }
 __global__ void k_route_rest_jobs(JobGrid J) {
@@ -612,6 +613,7 @@ __device__ __forceinline__ void k_round_prep_body(const BState& S, unsigned bx, 
                       S.samp_scratch ? S.samp_scratch + (size_t)k * S.F : nullptr);
 }
 __global__ void __launch_bounds__(PREP_THREADS) k_round_prep(BState S) {
+  follow_launch();
   k_round_prep_body(S, blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(PREP_THREADS) k_round_prep_jobs(JobGrid J) {
@@ -649,6 +651,7 @@ __device__ __forceinline__ void k_quantize_body(const BState& S, unsigned bx, un
   if (threadIdx.x < 2 && s_e[threadIdx.x]) atomicMax((unsigned int*)&S.qerr[0] + threadIdx.x, s_e[threadIdx.x]);
 }
 __global__ void k_quantize(BState S) {
+  follow_launch();
   k_quantize_body(S, blockIdx.x, gridDim.x);
 }
 __global__ void k_quantize_jobs(JobGrid J) {
@@ -1572,6 +1575,7 @@ __device__ __forceinline__ void k_eval_body(const BState& S, unsigned bx, int d)
   write_split(S, ni, best, cf >= 0, b);
 }
 __global__ void __launch_bounds__(EVAL_THREADS) k_eval(BState S, int d) {
+  follow_launch();
   k_eval_body(S, blockIdx.x, d);
 }
 __global__ void __launch_bounds__(EVAL_THREADS) k_eval_jobs(JobGrid J, int d) {
@@ -1765,6 +1769,7 @@ __device__ __forceinline__ void k_assign_body(const BState& S, unsigned bx, unsi
   }
 }
 __global__ void __launch_bounds__(1024) k_assign(BState S, int d, int write_tiles) {
+  follow_launch();
   k_assign_body(S, blockIdx.x, gridDim.x, d, write_tiles);
 }
 __global__ void __launch_bounds__(1024) k_assign_jobs(JobGrid J, int d, int write_tiles) {
@@ -1897,6 +1902,7 @@ __device__ __forceinline__ void k_partition_body(const BState& S, unsigned bx, u
   }
 }
 __global__ void __launch_bounds__(PART_THREADS, 4) k_partition(BState S, int d) {
+  follow_launch();
   k_partition_body(S, blockIdx.x, gridDim.x, d);
 }
 __global__ void __launch_bounds__(PART_THREADS, 4) k_partition_jobs(JobGrid J, int d) {
@@ -2000,6 +2006,7 @@ __device__ __forceinline__ void k_plan_body(const BState& S, unsigned bx, unsign
   }
 }
 __global__ void __launch_bounds__(1024) k_plan(BState S, int d) {
+  follow_launch();
   k_plan_body(S, blockIdx.x, gridDim.x, d);
 }
 __global__ void __launch_bounds__(1024) k_plan_jobs(JobGrid J, int d) {
@@ -2019,6 +2026,7 @@ __global__ void __launch_bounds__(1024) k_plan_jobs(JobGrid J, int d) {
 // sift_down_to_bottom and sift_up on pop), run by one thread on a
 // shared-memory copy of the queue, so equal keys leave in the same order.
 __global__ void __launch_bounds__(256) k_lg_heap(BState S, int init) {
+  follow_launch();
   extern __shared__ HeapEnt sh_heap[];  // [maxn]
   __shared__ int s_size;
   const int k = blockIdx.x, tid = threadIdx.x;
@@ -2113,6 +2121,7 @@ __global__ void __launch_bounds__(256) k_lg_heap(BState S, int init) {
 
 // The expanded node's partitioned rows back into the tree's row list.
 __global__ void k_lg_copy(BState S) {
+  follow_launch();
   const int ntiles = min(*S.ptile_count, S.ptile_cap);
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tile = S.ptiles[t];
@@ -2124,6 +2133,7 @@ __global__ void k_lg_copy(BState S) {
 // Leaf values of every leaf (hist.rs:193-200 then scale_leaves) and the
 // leaf value of each of its rows (the margin update, train.rs:326-328).
 __global__ void k_lg_finalize(BState S) {
+  follow_launch();
   const int k = blockIdx.y, nid = blockIdx.x;
   if (nid >= S.num_nodes[k]) return;
   const size_t ni = NI(S, k, nid);
@@ -2154,6 +2164,7 @@ __global__ void k_lg_finalize(BState S) {
 // The decisions are the partition's: missing -> default direction,
 // categorical -> the node's category set, numeric -> local bin <= split bin.
 __global__ void k_lg_route(BState S) {
+  follow_launch();
   const unsigned long long round = *S.round;
   const int K = S.K;
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (size_t)gridDim.x * blockDim.x) {
@@ -2202,6 +2213,7 @@ __device__ __forceinline__ void k_round_end_body(const BState& S, unsigned bx, u
   }
 }
 __global__ void k_round_end(BState S) {
+  follow_launch();
   k_round_end_body(S, blockIdx.x, gridDim.x);
 }
 __global__ void k_round_end_jobs(JobGrid J) {
@@ -2812,8 +2824,8 @@ int booster_round_body(sb_booster* b, int apply_delta) {
   S.apply_delta = apply_delta;
   SB_LAUNCH(ctx, k_gradient, gblocks, 256, 0, S);
   S.apply_delta = 0;
-  SB_LAUNCH(ctx, k_round_prep, (unsigned)b->K, PREP_THREADS, 0, S);
-  if (S.fixed) SB_LAUNCH(ctx, k_quantize, gblocks, 256, 0, S);
+  SB_LAUNCH_NEXT(ctx, k_round_prep, (unsigned)b->K, PREP_THREADS, 0, S);
+  if (S.fixed) SB_LAUNCH_NEXT(ctx, k_quantize, gblocks, 256, 0, S);
   HistLaunch L;
   L.g = b->g;
   L.gpair = S.fixed ? (const void*)S.gpk : (const void*)S.gpair;
@@ -2852,44 +2864,44 @@ int booster_round_body(sb_booster* b, int apply_delta) {
     const unsigned fy = (unsigned)((b->g->F + SCAN_WARPS - 1) / SCAN_WARPS);
     const size_t heap_smem = (size_t)b->maxn * sizeof(HeapEnt);
     auto eval = [&](int d, unsigned width) -> int {
-      SB_LAUNCH(ctx, k_eval, dim3(width, fy, (unsigned)b->K), EVAL_THREADS, esm, S, d);
+      SB_LAUNCH_NEXT(ctx, k_eval, dim3(width, fy, (unsigned)b->K), EVAL_THREADS, esm, S, d);
       return SB_OK;
     };
     SB_TRY(eval(0, 1));  // the root
-    SB_LAUNCH(ctx, k_lg_heap, (unsigned)b->K, 256, heap_smem, S, 1);
+    SB_LAUNCH_NEXT(ctx, k_lg_heap, (unsigned)b->K, 256, heap_smem, S, 1);
     // a step partitions one node per class tree: its tiles, at most
     const unsigned pblocks = part_blocks(ctx, b->n, b->K, b->K);
     for (int step = 0; step < b->steps; ++step) {
       const int d = step == 0 ? 0 : 1;  // only the first expansion reads the shared root list
-      SB_LAUNCH(ctx, k_assign, assign_blocks(b, 256), 256, 0, S, d, 1);  // one frontier node per tree
-      SB_LAUNCH(ctx, k_partition, pblocks, PART_THREADS, 0, S, d);
-      SB_LAUNCH(ctx, k_lg_copy, pblocks, 256, 0, S);
-      SB_LAUNCH(ctx, k_plan, 1, 1024, 0, S, d);
+      SB_LAUNCH_NEXT(ctx, k_assign, assign_blocks(b, 256), 256, 0, S, d, 1);  // one frontier node per tree
+      SB_LAUNCH_NEXT(ctx, k_partition, pblocks, PART_THREADS, 0, S, d);
+      SB_LAUNCH_NEXT(ctx, k_lg_copy, pblocks, 256, 0, S);
+      SB_LAUNCH_NEXT(ctx, k_plan, 1, 1024, 0, S, d);
       SB_TRY(hist(b->K));
       SB_TRY(eval(1, 2));
-      SB_LAUNCH(ctx, k_lg_heap, (unsigned)b->K, 256, heap_smem, S, 0);
+      SB_LAUNCH_NEXT(ctx, k_lg_heap, (unsigned)b->K, 256, heap_smem, S, 0);
     }
-    SB_LAUNCH(ctx, k_lg_finalize, dim3((unsigned)b->maxn, (unsigned)b->K), 256, 0, S);
-    if (!S.row_leaf && S.update_margin) SB_LAUNCH(ctx, k_lg_route, gblocks, 256, 0, S);
+    SB_LAUNCH_NEXT(ctx, k_lg_finalize, dim3((unsigned)b->maxn, (unsigned)b->K), 256, 0, S);
+    if (!S.row_leaf && S.update_margin) SB_LAUNCH_NEXT(ctx, k_lg_route, gblocks, 256, 0, S);
   }
   for (int d = 0; d < b->D && !b->lossguide; ++d) {
     const unsigned width = (unsigned)std::min(1 << d, b->maxw);
     dim3 sg(width, (unsigned)((b->g->F + SCAN_WARPS - 1) / SCAN_WARPS), (unsigned)b->K);
-    SB_LAUNCH(ctx, k_eval, sg, EVAL_THREADS, esm, S, d);
+    SB_LAUNCH_NEXT(ctx, k_eval, sg, EVAL_THREADS, esm, S, d);
     // 1024 threads: the threads also write the level's partition tiles (about
     // n / PART_TILE at the root), one binary search each
-    SB_LAUNCH(ctx, k_assign, assign_blocks(b, 1024), 1024, 0, S, d, 1);
+    SB_LAUNCH_NEXT(ctx, k_assign, assign_blocks(b, 1024), 1024, 0, S, d, 1);
     const unsigned pblocks = part_blocks(ctx, b->n, b->K, (size_t)b->K * width);
-    SB_LAUNCH(ctx, k_partition, pblocks, PART_THREADS, 0, S, d);
+    SB_LAUNCH_NEXT(ctx, k_partition, pblocks, PART_THREADS, 0, S, d);
     if (d + 1 < b->D) {
-      SB_LAUNCH(ctx, k_plan, 1, 1024, 0, S, d);
+      SB_LAUNCH_NEXT(ctx, k_plan, 1, 1024, 0, S, d);
       SB_TRY(hist(b->K * (1 << d)));
     }
   }
   // the rows outside the subset take their leaf values by routing (lossguide
   // rounds without row -> leaf output routed every row above)
-  if (!b->lossguide || S.row_leaf) SB_LAUNCH(ctx, k_route_rest, gblocks, 256, 0, S);
-  SB_LAUNCH(ctx, k_round_end, 1, 32, 0, S);
+  if (!b->lossguide || S.row_leaf) SB_LAUNCH_NEXT(ctx, k_route_rest, gblocks, 256, 0, S);
+  SB_LAUNCH_NEXT(ctx, k_round_end, 1, 32, 0, S);
   if (b->timing) {
     SB_CUDA(cudaEventRecord(r1, ctx->stream));
     b->ev.push_back(r0);

@@ -96,17 +96,17 @@ __device__ __forceinline__ void add_pair(unsigned a, unsigned hoff, uint32_t vg,
 // are meant to overlap (the compiler otherwise sinks them towards their use).
 __device__ __forceinline__ uint2 gather(const uint2* p) {
   uint2 v;
-  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint16_t gather(const uint16_t* p) {
   uint16_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint32_t gather(const uint32_t* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 
@@ -408,6 +408,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
 
 template <bool FIXED, int KIND, int RL, int THREADS = HIST_THREADS>
 __global__ void __launch_bounds__(THREADS, HIST_THREADS / THREADS) k_hist(HistDev a) {
+  follow_launch();
   hist_body<FIXED, KIND, RL>(a, blockIdx.x, gridDim.x);
 }
 
@@ -550,8 +551,8 @@ __device__ __forceinline__ void zero_items_body(const HistItem* items, const int
     reinterpret_cast<unsigned long long*>(items[it].total)[threadIdx.x] = 0ull;
 }
 
-__global__ void k_zero_items(const HistItem* __restrict__ items, const int* __restrict__ count, size_t words,
-                             HistParts parts) {
+__global__ void k_zero_items(const HistItem* items, const int* count, size_t words, HistParts parts) {
+  follow_launch();
   zero_items_body(items, count, words, parts, blockIdx.x, gridDim.x);
 }
 
@@ -903,7 +904,7 @@ int launch_hist(sb_ctx* ctx, const HistLaunch& L) {
   const int grid = hist_grid(ctx, L.g, L.rows_bound, L.rows_per_cta);
   const size_t sm = L.g->hist_smem_bytes;
   void (*kern)(HistDev) = reinterpret_cast<void (*)(HistDev)>(const_cast<void*>(hist_kernel(L.g, L.fixed != 0)));
-  SB_LAUNCH(ctx, kern, grid, L.g->hist_threads, sm, a);
+  SB_LAUNCH_NEXT(ctx, kern, grid, L.g->hist_threads, sm, a);
   return SB_OK;
 }
 
@@ -923,7 +924,7 @@ int launch_zero_items(sb_ctx* ctx, const HistLaunch& L) {
   if (L.max_items <= 0) return SB_OK;
   const size_t words = (L.g->total_bins + L.g->F) * 2;
   dim3 grid((unsigned)std::min<size_t>((words + 255) / 256, 64), (unsigned)L.max_items + 1);
-  SB_LAUNCH(ctx, k_zero_items, grid, ZERO_THREADS, 0, L.items, L.count, words, hist_parts(ctx, L));
+  SB_LAUNCH_NEXT(ctx, k_zero_items, grid, ZERO_THREADS, 0, L.items, L.count, words, hist_parts(ctx, L));
   return SB_OK;
 }
 
