@@ -135,7 +135,7 @@ struct BState {
   int* num_nodes;
   int* cat_count;
   // rows
-  uint32_t* rows0;          // [K][n]
+  uint32_t* rows0;          // [K][n]; the first n: the root list
   uint32_t* rows1;          // [K][n]
   unsigned int* kept;       // sampled rows this round (the root list's front)
   unsigned int* unkept;     // rows outside the subset (the root list's back)
@@ -191,6 +191,13 @@ __device__ __forceinline__ char* level_hist(const BState& S, int d, int k, int s
 
 __device__ __forceinline__ char* node_hist(const BState& S, int k, int nid) {
   return S.nhist + NI(S, k, nid) * (size_t)S.HB * 16;
+}
+
+// Tree k's row list of the nodes of odd or even depth. The nodes of a tree hold
+// disjoint parts of a list, so a partition reads one and writes the other
+// (a lossguide step used to copy the node's part back: 5 us of its 155).
+__device__ __forceinline__ uint32_t* node_rows(const BState& S, int k, int odd) {
+  return (odd ? S.rows1 : S.rows0) + (size_t)k * S.n;
 }
 
 // Histogram of frontier slot `slot` of tree k at level d (lossguide: of the node).
@@ -1792,9 +1799,6 @@ __device__ __forceinline__ void k_partition_body(const BState& S, unsigned bx, u
   __shared__ unsigned int s_base[2];
   const bool last = !S.lossguide && (d + 1 == S.max_depth);
   const int ntiles = min(*S.ptile_count, S.ptile_cap);
-  // lossguide: from the tree's list into the scratch list (k_lg_copy moves it back)
-  const uint32_t* rows_cur_all = (!S.lossguide && (d & 1)) ? S.rows1 : S.rows0;
-  uint32_t* rows_nxt_all = (!S.lossguide && (d & 1)) ? S.rows0 : S.rows1;
   const int K = S.K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
@@ -1802,8 +1806,10 @@ __device__ __forceinline__ void k_partition_body(const BState& S, unsigned bx, u
     const int4 tile = S.ptiles[t];
     const int k = tile.x, nid = tile.y;
     const size_t ni = NI(S, k, nid);
-    const uint32_t* rows_cur = rows_cur_all + (d == 0 ? 0 : (size_t)k * S.n);
-    uint32_t* rows_nxt = rows_nxt_all + (size_t)k * S.n;
+    // a node's rows lie in the list of its depth's parity, its children's in the other
+    const int odd = (S.lossguide ? S.ndepth[ni] : d) & 1;
+    const uint32_t* rows_cur = d == 0 ? S.rows0 : node_rows(S, k, odd);
+    uint32_t* rows_nxt = node_rows(S, k, odd ^ 1);
     if (!S.split[ni].valid) {  // a final leaf: its rows take the leaf value
       const float lv = S.leafval[ni];
       for (int p = tile.z + threadIdx.x; p < tile.w; p += PART_THREADS) {
@@ -1917,34 +1923,32 @@ __device__ __forceinline__ void k_plan_body(const BState& S, unsigned bx, unsign
   constexpr int GROUP = 1024;  // class trees per pass over the (tree, node) pairs
   __shared__ int sm_i[33];
   __shared__ unsigned long long sm_u[33];
-  __shared__ int s_items;
-  __shared__ unsigned long long s_pos;
   __shared__ int s_off[GROUP + 1];
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    s_items = 0;
-    s_pos = 0;
-  }
-  __syncthreads();
+  int items = 0;  // the same in every thread, as is pos
+  unsigned long long pos = 0;
   const unsigned long long round = *S.round;
   const int dn = d + 1;
   for (int k0 = 0; k0 < S.K; k0 += GROUP) {
     const int nk = min(GROUP, S.K - k0);
     // offsets of the group's frontiers in its list of (tree, node) pairs
-    int base = 0;  // the same in every thread
-    for (int j0 = 0; j0 < nk; j0 += blockDim.x) {
-      const int j = j0 + tid;
-      int tot;
-      const int o = block_scan_excl<int>(j < nk ? S.prev_count[k0 + j] : 0, &tot, sm_i);
-      if (j < nk) s_off[j] = base + o;
-      base += tot;
+    int pairs = 0;  // the same in every thread
+    if (nk == 1) {
+      pairs = S.prev_count[k0];
+    } else {
+      for (int j0 = 0; j0 < nk; j0 += blockDim.x) {
+        const int j = j0 + tid;
+        int tot;
+        const int o = block_scan_excl<int>(j < nk ? S.prev_count[k0 + j] : 0, &tot, sm_i);
+        if (j < nk) s_off[j] = pairs + o;
+        pairs += tot;
+      }
+      __syncthreads();
     }
-    if (tid == 0) s_off[nk] = base;
-    __syncthreads();
-    const int pairs = s_off[nk];
     for (int c0 = 0; c0 < pairs; c0 += blockDim.x) {
       const int q = c0 + tid;
       int v = 0, k = k0, bchild = -1;
+      const uint32_t* rows = nullptr;
       unsigned long long len = 0;
       uint2 bseg = make_uint2(0, 0);
       if (q < pairs) {
@@ -1954,34 +1958,37 @@ __device__ __forceinline__ void k_plan_body(const BState& S, unsigned bx, unsign
           if (s_off[mid] <= q) lo = mid; else hi = mid;
         }
         k = k0 + lo;
-        const int nid = S.prev_begin[k] + (q - s_off[lo]);
+        const int nid = S.prev_begin[k] + (nk == 1 ? q : q - s_off[lo]);
         const size_t ni = NI(S, k, nid);
-        if (S.split[ni].valid) {
-          const sb_node* out = S.out_nodes + ((size_t)round * S.K + k) * S.maxn;
-          const Fill fl = S.fill[ni];
-          const uint2 sg = S.seg[ni];
-          const int l = out[nid].left, r = l + 1;
+        // asked for together
+        const int split = S.split[ni].valid, l = S.out_nodes[((size_t)round * S.K + k) * S.maxn + nid].left;
+        const Fill fl = S.fill[ni];
+        const uint2 sg = S.seg[ni];
+        rows = node_rows(S, k, (S.lossguide ? S.ndepth[ni] + 1 : dn) & 1);
+        if (split) {
+          const int r = l + 1;
           const size_t li = NI(S, k, l), ri = NI(S, k, r);
-          S.seg[li] = make_uint2(sg.x, sg.x + fl.left);
-          S.seg[ri] = make_uint2(sg.x + fl.left, sg.y);
+          const uint2 ls = make_uint2(sg.x, sg.x + fl.left), rs = make_uint2(sg.x + fl.left, sg.y);
+          S.seg[li] = ls;
+          S.seg[ri] = rs;
           S.nsamp[li] = fl.left;
           S.nsamp[ri] = fl.right;
           const bool build_left = fl.left <= fl.right;
           S.built[li] = build_left ? 1 : 0;
           S.built[ri] = build_left ? 0 : 1;
           bchild = build_left ? l : r;
-          bseg = build_left ? S.seg[li] : S.seg[ri];
+          bseg = build_left ? ls : rs;
           v = 1;
           len = bseg.y - bseg.x;
         }
       }
-      int tot_v;
-      const int idx = s_items + block_scan_excl<int>(v, &tot_v, sm_i);
-      unsigned long long tot_len;
-      const unsigned long long pos = s_pos + block_scan_excl<unsigned long long>(len, &tot_len, sm_u);
+      // items and rows before the pair: 11 and 53 bits
+      unsigned long long tot;
+      const unsigned long long at = block_scan_excl<unsigned long long>((unsigned long long)v | len << 11, &tot, sm_u);
+      const int idx = items + (int)(at & 0x7FFu);
       if (v) {
         HistItem it;
-        it.rows = ((!S.lossguide && (dn & 1)) ? S.rows1 : S.rows0) + (size_t)k * S.n;
+        it.rows = rows;
         it.begin = bseg.x;
         it.end = bseg.y;
         it.k = (uint32_t)k;
@@ -1989,19 +1996,16 @@ __device__ __forceinline__ void k_plan_body(const BState& S, unsigned bx, unsign
         it.out = S.lossguide ? node_hist(S, k, bchild) : level_hist(S, dn, k, bchild - S.lvl_begin[k]);
         it.total = nullptr;
         S.items[idx] = it;
-        S.prefix[idx] = pos;
+        S.prefix[idx] = pos + (at >> 11);
       }
-      __syncthreads();
-      if (tid == 0) {
-        s_items += tot_v;
-        s_pos += tot_len;
-      }
-      __syncthreads();
+      items += (int)(tot & 0x7FFu);
+      pos += tot >> 11;
     }
+    __syncthreads();  // s_off is written again
   }
   if (tid == 0) {
-    *S.item_count = s_items;
-    S.prefix[s_items] = s_pos;
+    *S.item_count = items;
+    S.prefix[items] = pos;
     *S.ptile_count = 0;  // the partition has consumed this level's tiles
   }
 }
@@ -2119,17 +2123,6 @@ __global__ void __launch_bounds__(256) k_lg_heap(BState S, int init) {
   if (tid == 0) S.heap_size[k] = size1;
 }
 
-// The expanded node's partitioned rows back into the tree's row list.
-__global__ void k_lg_copy(BState S) {
-  follow_launch();
-  const int ntiles = min(*S.ptile_count, S.ptile_cap);
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int4 tile = S.ptiles[t];
-    const size_t base = (size_t)tile.x * S.n;
-    for (int p = tile.z + threadIdx.x; p < tile.w; p += blockDim.x) S.rows0[base + p] = S.rows1[base + p];
-  }
-}
-
 // Leaf values of every leaf (hist.rs:193-200 then scale_leaves) and the
 // leaf value of each of its rows (the margin update, train.rs:326-328).
 __global__ void k_lg_finalize(BState S) {
@@ -2147,7 +2140,7 @@ __global__ void k_lg_finalize(BState S) {
   }
   if (!S.row_leaf) return;  // k_lg_route gives every row its leaf values
   const uint2 sg = S.seg[ni];
-  const uint32_t* rows = S.rows0 + (nid == 0 ? 0 : (size_t)k * S.n);  // an unsplit root keeps the shared list
+  const uint32_t* rows = node_rows(S, k, S.ndepth[ni] & 1);  // one tree: row -> leaf output is single-tree
   for (uint32_t p = sg.x + threadIdx.x; p < sg.y; p += blockDim.x) {
     const uint32_t rv = rows[p];
     const uint32_t id = rv & ~UNSAMPLED;
@@ -2875,7 +2868,6 @@ int booster_round_body(sb_booster* b, int apply_delta) {
       const int d = step == 0 ? 0 : 1;  // only the first expansion reads the shared root list
       SB_LAUNCH_NEXT(ctx, k_assign, assign_blocks(b, 256), 256, 0, S, d, 1);  // one frontier node per tree
       SB_LAUNCH_NEXT(ctx, k_partition, pblocks, PART_THREADS, 0, S, d);
-      SB_LAUNCH_NEXT(ctx, k_lg_copy, pblocks, 256, 0, S);
       SB_LAUNCH_NEXT(ctx, k_plan, 1, 1024, 0, S, d);
       SB_TRY(hist(b->K));
       SB_TRY(eval(1, 2));
