@@ -382,10 +382,11 @@ struct DevEnsemble {
   int shap_max_fc = 1;       // most distinct features in one chunk
   bool shap_valid = false;   // the TreeSHAP state above has been built (shap_prepare)
   bool shap_table = false;   // per-path contribution tables are in use
-  DBuf<float> shap_tab;      // per path: [2^D][round_up(D, 4)] f32 contributions
-  DBuf<long long> shap_tab_off;  // [n_paths] first float of each path's table
+  DBuf<float> shap_tab;      // per table: [2^elements][round_up(D, 4)] f32 contributions of a leaf or two siblings
+  DBuf<long long> shap_tab_off;  // first float of each table
+  DBuf<int> tree_tab;        // [n_trees + 1] each tree's tables
   DBuf<int4> tab_el;         // per element: {feature, lo, hi, (table-chunk feature index << 1) | miss_ok}
-  DBuf<int4> tab_head;       // per path: {first element, elements, table offset low, high 32 bits}
+  DBuf<int4> tab_head;       // per table: {first element, features | TAB_PAIR, table offset low, high 32 bits}
   DBuf<int4> tab_chunk;      // {class, first tree, trees, -}: work units of the table kernel
   DBuf<int> tab_chunk_fo;    // [n_tab_chunks + 1] offsets into tab_chunk_f
   DBuf<int> tab_chunk_f;     // each table chunk's distinct features
