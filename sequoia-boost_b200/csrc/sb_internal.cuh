@@ -368,7 +368,7 @@ struct DevEnsemble {
   DBuf<int64_t> tree_off;    // node offset per tree
   DBuf<uint32_t> cats;
   DBuf<float> weights;
-  DBuf<double> tree_mean;
+  std::vector<double> tree_mean;  // node_mean_value of each root, with the TreeSHAP state
   // TreeSHAP: the root-to-leaf paths of every tree
   DBuf<PathEl> path_el;      // elements, path after path
   DBuf<int> path_off;        // [n_paths + 1] element offsets

@@ -307,7 +307,7 @@ int model_upload(sb_model* m) {
   std::vector<int64_t> off(T + 1, 0);
   for (int t = 0; t < T; ++t) off[t + 1] = off[t] + (int64_t)m->trees[t].nodes.size();
   std::vector<int4> packed(off[T]);
-  std::vector<int> catend(off[T], 0);
+  std::vector<int> catend;  // empty without categorical nodes: nothing reads it then
   std::vector<uint32_t> cats;
   int maxd = 0;
   bool compact = off[T] > 0;  // every tree has the 8-byte form (CN_*)
@@ -328,6 +328,7 @@ int model_upload(sb_model* m) {
         std::memcpy(&x.y, &lv, 4);
       } else if (nd.is_categorical) {
         x.y = cat_base + (int)nd.cat_begin;
+        if (catend.empty()) catend.resize(off[T], 0);
         catend[off[t] + i] = cat_base + (int)nd.cat_end;
       } else {
         float c = nd.split_cond;
@@ -361,10 +362,6 @@ int model_upload(sb_model* m) {
   SB_TRY(D.cat_end.alloc(ctx, std::max<size_t>(catend.size(), 1)));
   if (!catend.empty())
     SB_CUDA(cudaMemcpyAsync(D.cat_end.p, catend.data(), catend.size() * 4, cudaMemcpyHostToDevice, st));
-  std::vector<double> means(T);
-  for (int t = 0; t < T; ++t) means[t] = node_mean_value(m->trees[t], 0);
-  SB_TRY(D.tree_mean.alloc(ctx, std::max(T, 1)));
-  if (T) SB_CUDA(cudaMemcpyAsync(D.tree_mean.p, means.data(), T * 8, cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaStreamSynchronize(st));
   D.n_trees = T;
   D.max_depth = maxd;

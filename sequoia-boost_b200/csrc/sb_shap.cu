@@ -990,6 +990,8 @@ int shap_prepare(sb_model* m) {
       SB_CUDA(cudaStreamSynchronize(st));  // the host vectors are released on return
     }
   }
+  D.tree_mean.resize(T);
+  for (int t = 0; t < T; ++t) D.tree_mean[t] = node_mean_value(m->trees[t], 0);
   SB_CUDA(cudaStreamSynchronize(st));
   D.shap_valid = true;
   return SB_OK;
@@ -1080,14 +1082,9 @@ int predict_contribs_device(sb_model* m, const float* d_X, size_t n, size_t F, f
   const int T = m->dev.n_trees;
   const size_t width = F + 1;
   // bias per class: base_score + sum of tree means in tree order (shap.rs:340-359)
-  std::vector<double> means(T);
-  if (T) {
-    SB_CUDA(cudaMemcpyAsync(means.data(), m->dev.tree_mean.p, T * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    SB_CUDA(cudaStreamSynchronize(ctx->stream));
-  }
   std::vector<double> bias(K, 0.0);
   for (int c = 0; c < K; ++c) bias[c] += (double)m->base_score;
-  for (int t = 0; t < T; ++t) bias[t % K] += means[t];
+  for (int t = 0; t < T; ++t) bias[t % K] += m->dev.tree_mean[t];
   DBuf<double> d_bias, acc;
   SB_TRY(d_bias.alloc(ctx, K));
   SB_CUDA(cudaMemcpyAsync(d_bias.p, bias.data(), K * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -1121,7 +1118,7 @@ int predict_interactions_device(sb_model* m, const float* d_X, size_t n, size_t 
   SB_TRY(raise_smem_limit((const void*)k_shap_inter<SHAP_INTER_MAXL>, smem));
   // [F][F] cell per class: the sum of its trees' expected values (shap.rs:427-437)
   std::vector<double> bias(K, 0.0);
-  for (int t = 0; t < T; ++t) bias[t % K] += node_mean_value(m->trees[t], 0);
+  for (int t = 0; t < T; ++t) bias[t % K] += m->dev.tree_mean[t];
   DBuf<double> d_bias, acc;
   SB_TRY(d_bias.alloc(ctx, K));
   SB_CUDA(cudaMemcpyAsync(d_bias.p, bias.data(), K * 8, cudaMemcpyHostToDevice, ctx->stream));
