@@ -529,6 +529,14 @@ constexpr int TAB_CHUNK_PATHS = 1024;  // leaves of a chunk
 constexpr int TAB_CHUNK_FEATURES = 192;  // distinct features of a chunk (its partial's rows)
 constexpr int TAB_TPR = 8;               // threads per row
 constexpr int TAB_ILP = 1;               // paths in flight per thread
+constexpr int TAB_BLOCKS = 2048 / (TAB_ROWS * TAB_TPR);  // blocks per SM
+// Blocks that share a chunk's tables, at most: each zeroes and flushes partials
+// of its own. Few rows make fewer blocks than the chip holds, and their time is
+// one block's chain of fetches (1000 trees of depth 8, whole calls: 3 rows 0.28
+// -> 0.18 ms, 40 rows 0.30 -> 0.20; 300 trees of depth 6, 512 rows 0.22 -> 0.17).
+// Chunks of half as many blocks for all requests, 2048 leaves instead of 1024:
+// 4096 rows 6.82 -> 6.71 ms, but 3 rows 0.30 -> 0.50.
+constexpr int TAB_MAX_PARTS = 8;
 
 // Shared memory of one k_shap_table block for a chunk of `nfc` features:
 // the f32 partials [nfc][TAB_ROWS] and the row values [nfc][TAB_STRIDE].
@@ -576,7 +584,7 @@ k_shap_table(ShapTabDev P, const float* __restrict__ X, size_t n, int F, float m
   for (int ti = 0; ti < ch.z; ++ti) {
     const int t = ch.y + ti * P.K;
     const int pe = P.tree_tab[t + 1];
-    for (int p0 = P.tree_tab[t] + grp * ILP; p0 < pe; p0 += TPR * ILP) {
+    for (int p0 = P.tree_tab[t] + (grp + blockIdx.y * TPR) * ILP; p0 < pe; p0 += TPR * ILP * gridDim.y) {
       // ILP paths at a time, every element loop unrolled to the table depth
       // limit, so that all their element and table loads are in flight
       // together; each element's chunk-feature index stays in a register for
@@ -1061,7 +1069,10 @@ int shap_paths(sb_model* m, cudaStream_t st, const float* d_X, size_t n, size_t 
     // 4096 rows of single-leaf tables 11.5 ms with the loops of 10, 10.7 ms with
     // those of 8)
     auto kern = L - 1 <= 8 ? k_shap_table<TAB_TPR, TAB_ILP, 8> : k_shap_table<TAB_TPR, TAB_ILP, SHAP_TABLE_MAXD>;
-    SB_LAUNCH_ON(ctx, st, kern, (unsigned)tb, TAB_ROWS * TAB_TPR, shap_table_smem(m->dev.tab_max_fc), Q, d_X, n,
+    // a chunk's tables are shared out over as many blocks as still run at once
+    const unsigned parts = (unsigned)std::max<unsigned long long>(
+        1, std::min<unsigned long long>(TAB_MAX_PARTS, (unsigned long long)ctx->num_sms * TAB_BLOCKS / tb));
+    SB_LAUNCH_ON(ctx, st, kern, dim3((unsigned)tb, parts), TAB_ROWS * TAB_TPR, shap_table_smem(m->dev.tab_max_fc), Q, d_X, n,
                  (int)F, missing, trb, d_acc);
   } else if (L <= 5) {
     SB_LAUNCH_ON(ctx, st, k_shap_paths<5>, grid, R, smem, P, d_X, n, (int)F, K, missing, row_blocks, d_acc);
