@@ -132,7 +132,9 @@ __device__ __forceinline__ uint32_t code_word(uint16_t v, int) { return v; }
 //    shared reduction compiles to a branch around it, which also keeps loads
 //    from moving ahead of adds (100 warp instructions per 100-feature row, 45
 //    without; LANES at 10M rows x 100 features, root level, per launch: 756 us
-//    with a test per row, 486 without);
+//    with a test per row, 486 without). FP32 tests each position: a shared f32
+//    reduction is a compare-and-swap loop, and warps that meet in a lane's
+//    unused word retry (10M rows x 100 features, per launch: 1.78 ms, 0.78 with the test);
 //  - LANES, whose 32 lanes hit 32 banks, needs 8 passes for 4 positions per
 //    lane where TILED's 25 lanes of random bins need 23.
 template <bool FIXED, int KIND, int RL>
@@ -192,6 +194,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
     // flush leaves out (LANES: entry 0 of its column).
     unsigned base[S];
     uint32_t keep[2] = {0, 0};  // code bits that count
+    unsigned pool = 0;          // FP32: the positions that are added
 #pragma unroll
     for (int j = 0; j < S; ++j) {
       int f = LANES ? a.slot_feat[pos0 + j] : pos0 + j;
@@ -199,6 +202,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
       const bool in_pool =
           f >= 0 && (!a.pool_mask || ((a.pool_mask[(size_t)item.k * a.FW + (f >> 5)] >> (f & 31)) & 1u));
       base[j] = sh_base;
+      pool |= (unsigned)in_pool << j;
       if (!in_pool) base[j] += 4u * (unsigned)(LANES ? lane : nent + lane);
       else if (U8) base[j] += 4u * (a.foff[f] - (unsigned)tile.bin0 + (unsigned)(4 * grp + j));
       if (in_pool) keep[U8 ? 0 : j >> 1] |= U8 ? 0xFFu << (8 * j) : 0xFFFFu << (16 * (j & 1));
@@ -262,7 +266,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
         for (int j = 0; j < S; ++j) {
           const uint32_t w = code_word(bv[q], U8 ? 0 : j >> 1) & keep[U8 ? 0 : j >> 1];
           const uint32_t c = U8 ? (w >> (8 * j)) & 0xFFu : (j & 1) ? w >> 16 : w & 0xFFFFu;
-          add_pair<FIXED>(base[j] + 4u * c, hoff, vg, vh);
+          if (FIXED || (pool >> j & 1)) add_pair<FIXED>(base[j] + 4u * c, hoff, vg, vh);
         }
       }
     };
