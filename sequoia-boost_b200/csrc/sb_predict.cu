@@ -165,10 +165,15 @@ __global__ void __launch_bounds__(LEAF_THREADS) k_leaf_values(PredDev P, const f
 // warps bring the next chunk's weighted values into shared memory while the
 // first min(K, 16) add the current one (warp w takes the classes c with c % 16
 // == w; lane = row).
-constexpr int SUM_ROWS = 32, SUM_WARPS = 16, SUM_CHUNK = 256;
+// The serving loop's blocks have 4 warps and 16 KB: beside a batch of
+// explanations an SM frees little at a time, and blocks of 16 warps waited for it
+// behind that batch (requests of at most 4096 rows, p99 24 ms).
+constexpr int SUM_ROWS = 32;
+template <int SUM_WARPS>
 __global__ void __launch_bounds__(SUM_ROWS * SUM_WARPS)
     k_margin_sum(PredDev P, const float* __restrict__ buf, size_t n, int K, int limit, MarginStart start, int objective,
                  float* __restrict__ out) {
+  constexpr int SUM_CHUNK = 16 * SUM_WARPS;
   extern __shared__ float sum_sm[];  // [2][SUM_CHUNK][SUM_ROWS]
   auto s_leaf = reinterpret_cast<float(*)[SUM_CHUNK][SUM_ROWS]>(sum_sm);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -228,10 +233,11 @@ __global__ void __launch_bounds__(SUM_ROWS * SUM_WARPS)
 }
 
 // n rows' margins on a stream; with transform_objective >= 0 a single output
-// is put through pred_transform as well. d_buf holds chunk * T floats.
+// is put through pred_transform as well. d_buf holds chunk * T floats. `serving`:
+// beside other kernels, in small blocks.
 int margins(sb_ctx* ctx, cudaStream_t st, const PredDev& P, const float* d_X, size_t n, size_t F, float missing,
             int K, int limit, float base, const float* d_bm, int bm_kind, float* d_buf, size_t chunk, float* d_out,
-            int transform_objective) {
+            int transform_objective, bool serving) {
   const int objective = K == 1 && transform_objective >= 0 ? transform_objective : (int)SB_OBJ_SQUARED_ERROR;
   for (size_t r0 = 0; r0 < n; r0 += chunk) {
     const size_t nb = std::min(chunk, n - r0);
@@ -249,9 +255,11 @@ int margins(sb_ctx* ctx, cudaStream_t st, const PredDev& P, const float* d_X, si
                    staged, per_thread, d_buf);
     }
     const float* bm = d_bm ? d_bm + (bm_kind == 1 ? r0 * K : r0) : nullptr;
-    constexpr size_t sum_smem = 2 * SUM_CHUNK * SUM_ROWS * sizeof(float);
-    SB_TRY(raise_smem_limit((const void*)k_margin_sum, sum_smem));
-    SB_LAUNCH_ON(ctx, st, k_margin_sum, (unsigned)((nb + SUM_ROWS - 1) / SUM_ROWS), SUM_ROWS * SUM_WARPS, sum_smem, P, d_buf, nb, K,
+    const int warps = serving ? 4 : 16;
+    const size_t sum_smem = 2 * 16 * warps * SUM_ROWS * sizeof(float);
+    auto sum = serving ? k_margin_sum<4> : k_margin_sum<16>;
+    SB_TRY(raise_smem_limit((const void*)sum, sum_smem));
+    SB_LAUNCH_ON(ctx, st, sum, (unsigned)((nb + SUM_ROWS - 1) / SUM_ROWS), SUM_ROWS * warps, sum_smem, P, d_buf, nb, K,
                  limit, MarginStart{base, bm, bm ? bm_kind : 0}, objective, d_out + r0 * K);
   }
   return SB_OK;
@@ -401,7 +409,7 @@ int predict_margin_device(sb_model* m, const float* d_X, size_t n, size_t F, flo
   DBuf<float> buf;
   if (limit > 0) SB_TRY(buf.alloc(ctx, (size_t)limit * chunk));
   return margins(ctx, ctx->stream, P, d_X, n, F, missing, Kc, limit, m->base_score, d_base_margin, bm_kind, buf.p,
-                 chunk, d_out, transform_objective);
+                 chunk, d_out, transform_objective, false);
 }
 
 // The margins of n host rows, through their device buffer d_X. Many rows go in
@@ -455,7 +463,7 @@ int margin_batch(sb_model* m, cudaStream_t st, const float* d_X, size_t n, size_
   const PredDev P = pred_dev(m);
   if (n == 0) return SB_OK;
   return margins(ctx, st, P, d_X, n, F, missing, Kc, m->dev.n_trees, m->base_score, nullptr, 0, d_buf, buf_rows,
-                 d_out, -1);
+                 d_out, -1, true);
 }
 
 }  // namespace sb
