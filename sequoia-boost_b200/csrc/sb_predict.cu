@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(LEAF_THREADS) k_leaf_values(PredDev P, const f
 // == w; lane = row).
 // The serving loop's blocks have 4 warps and 16 KB: beside a batch of
 // explanations an SM frees little at a time, and blocks of 16 warps waited for it
-// behind that batch (requests of at most 4096 rows, p99 24 ms).
+// behind that batch (mixed stream, requests of at most 4096 rows: p99 24 ms, 0.9
+// with these).
 constexpr int SUM_ROWS = 32;
 template <int SUM_WARPS>
 __global__ void __launch_bounds__(SUM_ROWS * SUM_WARPS)
