@@ -39,10 +39,11 @@ __device__ __forceinline__ bool is_missing_d(float v, float missing, bool miss_n
   return miss_nan ? isnan(v) : (v == missing);
 }
 
-// RegTree::leaf_id_with over a dense row (regtree.rs:213-242): the leaf's
-// node index, and its packed node in *leaf.
-__device__ __forceinline__ int route_to_leaf(const PredDev& P, int t, const float* row, float missing,
-                                             bool miss_nan, int4* leaf) {
+// RegTree::leaf_id_with over a dense row (regtree.rs:213-242) whose value of
+// feature f is value(f): the leaf's node index, and its packed node in *leaf.
+template <typename Value>
+__device__ __forceinline__ int route_to_leaf(const PredDev& P, int t, float missing, bool miss_nan, Value value,
+                                             int4* leaf) {
   const int4* nd = P.nodes + P.tree_off[t];
   int nid = 0;
   for (;;) {
@@ -52,7 +53,7 @@ __device__ __forceinline__ int route_to_leaf(const PredDev& P, int t, const floa
       return nid;
     }
     uint32_t ff = (uint32_t)x.x;
-    float v = row[ff & NF_FEATURE];
+    float v = value(ff & NF_FEATURE);
     bool go_left;
     if (is_missing_d(v, missing, miss_nan)) {
       go_left = (ff & NF_DEFAULT_LEFT) != 0;
@@ -71,14 +72,6 @@ __device__ __forceinline__ int route_to_leaf(const PredDev& P, int t, const floa
   }
 }
 
-// The leaf value of one tree for a dense row.
-__device__ __forceinline__ float route(const PredDev& P, int t, const float* row, float missing,
-                                       bool miss_nan) {
-  int4 x;
-  route_to_leaf(P, t, row, missing, miss_nan, &x);
-  return __int_as_float(x.y);
-}
-
 // predict_leaf (model.rs:330-341): out [n][T] leaf node ids, one thread per
 // (row, tree) with the tree index fastest, so the stores are coalesced and a
 // warp reads one row.
@@ -89,8 +82,9 @@ __global__ void k_leaf_ids(PredDev P, const float* __restrict__ X, size_t n, int
   if (i >= n * T) return;
   const size_t r = i / T;
   const int t = (int)(i - r * T);
+  const float* row = X + r * F;
   int4 x;
-  out[i] = (uint32_t)route_to_leaf(P, t, X + r * F, missing, isnan(missing), &x);
+  out[i] = (uint32_t)route_to_leaf(P, t, missing, isnan(missing), [&](uint32_t f) { return row[f]; }, &x);
 }
 
 // The leaf value of a tree in compact nodes `nd` for a row whose value of
@@ -119,15 +113,15 @@ __device__ __forceinline__ float margin_start(const MarginStart& m, size_t r, in
 }
 
 // Margins in two phases. Phase 1: the leaf value of every (row, tree),
-// tree-major. A block takes 2^lr >= min(n, 32) rows, their values staged in
-// shared memory (read row by row from global memory they cost a sector per
-// value), and a tree per remaining thread, so that all trees of a small
-// request are walked at once: its time is one tree's chain of dependent loads.
-// With many rows a thread takes up to 8 trees per staged row, and the time is
-// the gathers of nodes, 8 bytes each (16 rows x 1000 trees of depth 8: 8.9 ->
-// 5.2 us; 65,536 rows: 1.85 -> 0.86 ms; one kernel that streams the nodes
-// through shared memory and adds in place took 0.85 ms for both phases there
-// and 0.12 ms for any small request).
+// tree-major. A block takes 2^lr >= min(n, 32) rows and a tree per remaining
+// thread, so that all trees of a small request are walked at once: its time is
+// one tree's chain of dependent loads. With many rows a thread takes up to 8
+// trees and the block's rows are staged in shared memory (read row by row from
+// global memory they cost a sector per value); the time is then the gathers of
+// nodes, 8 bytes each (16 rows x 1000 trees of depth 8: 8.9 -> 5.2 us; 65,536
+// rows: 1.85 -> 0.86 ms; one kernel that streams the nodes through shared memory
+// and adds in place took 0.85 ms for both phases there and 0.12 ms for any small
+// request). Which rows are staged: leaf_plan.
 constexpr int LEAF_THREADS = 128;
 __global__ void __launch_bounds__(LEAF_THREADS) k_leaf_values(PredDev P, const float* __restrict__ X, size_t n, int F,
                                                               float missing, int limit, int lr, int staged,
@@ -147,15 +141,22 @@ __global__ void __launch_bounds__(LEAF_THREADS) k_leaf_values(PredDev P, const f
     __syncthreads();
   }
   if (r >= n) return;
+  const float* own = X + r * F;
+  auto global = [&](uint32_t f) { return own[f]; };
   for (int i = 0; i < per_thread; ++i) {
     const int t = t0 + i * tpb;
     if (t >= limit) return;
     float v;
-    if (P.cnodes && staged)
+    if (staged) {
       v = route_compact(P.cnodes + P.tree_off[t], missing, miss_nan,
                         [&](uint32_t f) { return s_rows[f * (rows + 1) + row]; });
-    else
-      v = route(P, t, X + r * F, missing, miss_nan);
+    } else if (P.cnodes) {
+      v = route_compact(P.cnodes + P.tree_off[t], missing, miss_nan, global);
+    } else {
+      int4 x;
+      route_to_leaf(P, t, missing, miss_nan, global, &x);
+      v = __int_as_float(x.y);
+    }
     buf[(size_t)t * n + r] = v;
   }
 }
@@ -233,6 +234,36 @@ __global__ void __launch_bounds__(SUM_ROWS * SUM_WARPS)
   if (warp < K) out[r * K + warp] = acc;
 }
 
+// Rows and trees of a k_leaf_values block.
+struct LeafPlan {
+  int lr, staged, per_thread;
+  size_t smem;
+};
+// Staged rows are paid for by what is read of them: a copy of all F values
+// against about a path of each of the block's trees. Whole calls, staged /
+// read from global memory, us: 4096 rows x 100 features x 1000 trees of depth 8
+// (32 trees to a block) 206 / 227; 300 rows (4 trees) 86 / 75; 1000 rows x 360
+// features x 500 trees of depth 6 194 / 139. 16-byte nodes read from global
+// memory at any size, since their walk leaves L1 to the rows (4096 rows x 100
+// features, 500 trees of depth 8 with categorical splits: 464 staged, 362 not). Without staging a thread takes one tree: more of them only leave an
+// uneven last wave (the same call: 362 at up to 8 trees, 301 at one).
+LeafPlan leaf_plan(size_t n, size_t F, size_t limit, bool compact, int num_sms) {
+  LeafPlan p{0, 0, 1, 0};
+  while (p.lr < 5 && ((size_t)1 << p.lr) < n) ++p.lr;
+  // one tree per thread while all fit the chip at once, up to 8
+  const size_t pairs = n * limit, chip = (size_t)num_sms * 2048;
+  const int many = (int)std::max<size_t>(1, std::min<size_t>(8, pairs / chip));
+  const size_t sm = F * sizeof(float) * ((1 << p.lr) + 1), trees = (size_t)(LEAF_THREADS >> p.lr) * many;
+  if (compact && sm <= 48 * 1024 && F <= 4 * trees) {
+    p.staged = 1;
+    p.per_thread = many;
+    p.smem = sm;
+  }
+  const size_t at_once = (size_t)(LEAF_THREADS >> p.lr) * 65535;  // a grid's rows of blocks
+  p.per_thread = std::max(p.per_thread, (int)((limit + at_once - 1) / at_once));
+  return p;
+}
+
 // n rows' margins on a stream; with transform_objective >= 0 a single output
 // is put through pred_transform as well. d_buf holds chunk * T floats. `serving`:
 // beside other kernels, in small blocks.
@@ -243,17 +274,11 @@ int margins(sb_ctx* ctx, cudaStream_t st, const PredDev& P, const float* d_X, si
   for (size_t r0 = 0; r0 < n; r0 += chunk) {
     const size_t nb = std::min(chunk, n - r0);
     if (limit > 0) {
-      int lr = 0;
-      while (lr < 5 && (size_t)(1 << lr) < nb) ++lr;
-      const size_t sm = F * sizeof(float) * ((1 << lr) + 1);
-      const int staged = sm <= 48 * 1024;
-      // one tree per thread while all fit the chip at once, up to 8
-      const size_t pairs = nb * (size_t)limit, chip = (size_t)ctx->num_sms * 2048;
-      const int per_thread = (int)std::max<size_t>(1, std::min<size_t>(8, pairs / chip));
-      const int per = (LEAF_THREADS >> lr) * per_thread;
-      dim3 grid((unsigned)((nb + (1 << lr) - 1) >> lr), (unsigned)((limit + per - 1) / per));
-      SB_LAUNCH_ON(ctx, st, k_leaf_values, grid, LEAF_THREADS, staged ? sm : 0, P, d_X + r0 * F, nb, (int)F, missing, limit, lr,
-                   staged, per_thread, d_buf);
+      const LeafPlan L = leaf_plan(nb, F, (size_t)limit, P.cnodes != nullptr, ctx->num_sms);
+      const int per = (LEAF_THREADS >> L.lr) * L.per_thread;
+      dim3 grid((unsigned)((nb + (1 << L.lr) - 1) >> L.lr), (unsigned)((limit + per - 1) / per));
+      SB_LAUNCH_ON(ctx, st, k_leaf_values, grid, LEAF_THREADS, L.smem, P, d_X + r0 * F, nb, (int)F, missing, limit, L.lr,
+                   L.staged, L.per_thread, d_buf);
     }
     const float* bm = d_bm ? d_bm + (bm_kind == 1 ? r0 * K : r0) : nullptr;
     const int warps = serving ? 4 : 16;

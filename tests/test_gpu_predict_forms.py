@@ -1,0 +1,42 @@
+"""Margins on either side of the rules that choose how a request is walked:
+rows staged in shared memory or read from global memory (features against the
+trees of a block), 8- and 16-byte nodes, uploads whole or in parts, the width
+of the ordered sum. Compared bit for bit with sums in tree order over leaves
+found by a plain walk."""
+import numpy as np
+import pytest
+
+from test_gpu_predict_paths import _forest, _margins
+
+pytestmark = pytest.mark.gpu
+
+
+def _categorical(nodes, trees, f, rng):
+    """The right child of every root splits on a code set of the last feature."""
+    at = np.arange(trees) * 7 + 2
+    nodes["split_feature"][at] = f - 1
+    nodes["is_categorical"][at] = 1
+    nodes["cat_end"][at] = 3
+    return np.stack([rng.permutation(6)[:3] for _ in range(trees)]).astype(np.uint32)
+
+
+# one row walks 128 trees per block, 2 rows 64, 16 rows 8, from 17 on 4
+@pytest.mark.parametrize("n,f", [(1, 512), (1, 513), (2, 256), (2, 257), (16, 32), (16, 33), (33, 16), (33, 17)])
+@pytest.mark.parametrize("form", ["compact", "apart", "categorical"])
+def test_staging_and_node_forms(sb, ctx, n, f, form):
+    rng = np.random.default_rng(100 * n + f)
+    trees = 9
+    off, nodes = _forest(sb, rng, trees, f, form == "apart")
+    x = rng.standard_normal((n, f)).astype(np.float32)
+    cats, cat_off = np.zeros((trees, 0), np.uint32), np.zeros(trees + 1, np.int64)
+    if form == "categorical":
+        cats, cat_off = _categorical(nodes, trees, f, rng), np.arange(trees + 1, dtype=np.int64) * 3
+        x[:, f - 1] = rng.integers(0, 6, n)
+    x[rng.random(x.shape) < 0.2] = np.nan
+    m = sb.BoostedModel.from_arrays(off, nodes, cat_off, cats.reshape(-1), 0.25, 0, f, ctx=ctx)
+    from gpu_helpers import leaf_ids
+    want = np.full(n, np.float32(0.25), np.float32)
+    for t in range(trees):
+        nd = nodes[off[t]:off[t + 1]]
+        want = want + nd["leaf_value"][leaf_ids(nd, cats[t], x)]
+    assert np.array_equal(m.predict_margin(sb.DMatrix(x)), want)
