@@ -245,8 +245,9 @@ struct LeafPlan {
 // (32 trees to a block) 206 / 227; 300 rows (4 trees) 86 / 75; 1000 rows x 360
 // features x 500 trees of depth 6 194 / 139. 16-byte nodes read from global
 // memory at any size, since their walk leaves L1 to the rows (4096 rows x 100
-// features, 500 trees of depth 8 with categorical splits: 464 staged, 362 not). Without staging a thread takes one tree: more of them only leave an
-// uneven last wave (the same call: 362 at up to 8 trees, 301 at one).
+// features, 500 trees of depth 8 with categorical splits: 464 staged, 362 not).
+// Without staging a thread takes one tree: more of them only leave an uneven
+// last wave (the same call: 362 at up to 8 trees, 301 at one).
 LeafPlan leaf_plan(size_t n, size_t F, size_t limit, bool compact, int num_sms) {
   LeafPlan p{0, 0, 1, 0};
   while (p.lr < 5 && ((size_t)1 << p.lr) < n) ++p.lr;
@@ -438,18 +439,28 @@ int predict_margin_device(sb_model* m, const float* d_X, size_t n, size_t F, flo
                  chunk, d_out, transform_objective, false);
 }
 
-// The margins of n host rows, through their device buffer d_X. Many rows go in
-// parts, each copied on a second stream while the part before is computed
-// (65,536 rows x 100 features: 0.48 ms of copies beside 0.97 ms of kernels).
+// The margins of n host rows, through their device buffer d_X. Large requests
+// go in parts, each copied on a second stream while the part before is computed
+// (65,536 rows x 100 features, 1000 trees: 0.48 ms of copies beside 0.97 ms of
+// kernels). The stream, its event and the parts cost 0.05 to 0.15 ms, by the
+// host, so that both the copy and the walk have to take longer than that: from 4 MB
+// and 10 million (row, tree) pairs on. Whole calls in one part / in parts, ms:
+// 100,000 rows x 20, 60 trees 0.35 / 0.41; 20,000 rows x 100, 500 trees 0.61 / 0.56
+// on one host and 0.59 / 0.68 on another; 1000 trees 0.77 / 0.71; 65,536 rows x 20,
+// 500 trees 0.70 / 0.63; 1M rows x 20, 5 trees, pinned 2.4 / 2.9 (8192 rows to a
+// part). Eight parts at most: each copy starts anew (1M rows x 20, 300 trees: 122
+// parts 7.3, 8 parts 6.9).
 // The context's stream waits for every copy, so the buffers' order of use and
 // release on it is as with one stream.
-constexpr size_t PART_ROWS = 8192;
+constexpr size_t PART_ROWS = 8192, MAX_PARTS = 8;
+constexpr size_t SPLIT_BYTES = 4000000, SPLIT_PAIRS = 10000000;
 static int margins_from_host(sb_model* m, const float* X, float* d_X, size_t n, size_t F, float missing,
                              const float* d_base_margin, size_t ntree_limit, float* d_out, int transform_objective) {
   sb_ctx* ctx = m->ctx;
   const int K = m->num_class >= 2 ? m->num_class : 1;
   SB_TRY(model_upload(m));
-  if (n < 2 * PART_ROWS) {
+  const size_t trees = (size_t)m->dev.n_trees, limit = ntree_limit ? std::min(ntree_limit, trees) : trees;
+  if (n < 2 * PART_ROWS || n * F * sizeof(float) < SPLIT_BYTES || n * limit < SPLIT_PAIRS) {
     SB_CUDA(cudaMemcpyAsync(d_X, X, n * F * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     return predict_margin_device(m, d_X, n, F, missing, d_base_margin, 1, ntree_limit, d_out, transform_objective);
   }
@@ -468,8 +479,9 @@ static int margins_from_host(sb_model* m, const float* X, float* d_X, size_t n, 
   SB_CUDA(cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming));
   SB_CUDA(cudaEventRecord(s.ev, ctx->stream));  // d_X's allocation is ordered on the context's stream
   SB_CUDA(cudaStreamWaitEvent(s.st, s.ev, 0));
-  for (size_t r0 = 0; r0 < n; r0 += PART_ROWS) {
-    const size_t nb = std::min(PART_ROWS, n - r0);
+  const size_t part = std::max(PART_ROWS, (n + MAX_PARTS - 1) / MAX_PARTS);
+  for (size_t r0 = 0; r0 < n; r0 += part) {
+    const size_t nb = std::min(part, n - r0);
     SB_CUDA(cudaMemcpyAsync(d_X + r0 * F, X + r0 * F, nb * F * sizeof(float), cudaMemcpyHostToDevice, s.st));
     SB_CUDA(cudaEventRecord(s.ev, s.st));
     SB_CUDA(cudaStreamWaitEvent(ctx->stream, s.ev, 0));

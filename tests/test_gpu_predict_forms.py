@@ -6,6 +6,7 @@ found by a plain walk."""
 import numpy as np
 import pytest
 
+from gpu_helpers import leaf_ids
 from test_gpu_predict_paths import _forest, _margins
 
 pytestmark = pytest.mark.gpu
@@ -34,9 +35,27 @@ def test_staging_and_node_forms(sb, ctx, n, f, form):
         x[:, f - 1] = rng.integers(0, 6, n)
     x[rng.random(x.shape) < 0.2] = np.nan
     m = sb.BoostedModel.from_arrays(off, nodes, cat_off, cats.reshape(-1), 0.25, 0, f, ctx=ctx)
-    from gpu_helpers import leaf_ids
     want = np.full(n, np.float32(0.25), np.float32)
     for t in range(trees):
         nd = nodes[off[t]:off[t + 1]]
         want = want + nd["leaf_value"][leaf_ids(nd, cats[t], x)]
     assert np.array_equal(m.predict_margin(sb.DMatrix(x)), want)
+
+
+# (rows, features, trees, uploads): short of the bytes, of the pairs, and past both in 2 and in 8 parts
+@pytest.mark.parametrize("n,f,trees,parts", [(16_384, 61, 1000, 1), (16_384, 64, 610, 1), (16_385, 64, 611, 3),
+                                             (66_000, 40, 250, 8), (100_000, 20, 9, 1)])
+def test_uploads_in_parts(sb, ctx, n, f, trees, parts):
+    rng = np.random.default_rng(n + f)
+    off, nodes = _forest(sb, rng, trees, f)
+    x = rng.standard_normal((n, f)).astype(np.float32)
+    x[rng.random(x.shape) < 0.2] = np.nan
+    m = sb.BoostedModel.from_arrays(off, nodes, np.zeros(trees + 1, np.int64), [], 0.25, 0, f, ctx=ctx)
+    d = sb.DMatrix(x)
+    m.predict_margin(d)
+    before = ctx.launch_count()
+    got = m.predict_margin(d)
+    assert ctx.launch_count() - before == 2 * parts  # leaf values and sum of each part
+    some = np.unique(np.concatenate([[0, n - 1], np.arange(8_190, 8_194), np.arange(16_382, min(n, 16_386)),
+                                     rng.integers(0, n, 20)]))
+    assert np.array_equal(got[some], _margins(off, nodes, x[some], 0.25, 1, trees))
