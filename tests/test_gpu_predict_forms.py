@@ -59,3 +59,16 @@ def test_uploads_in_parts(sb, ctx, n, f, trees, parts):
     some = np.unique(np.concatenate([[0, n - 1], np.arange(8_190, 8_194), np.arange(16_382, min(n, 16_386)),
                                      rng.integers(0, n, 20)]))
     assert np.array_equal(got[some], _margins(off, nodes, x[some], 0.25, 1, trees))
+
+
+@pytest.mark.parametrize("k,trees", [(1, 64), (1, 65), (2, 63), (4, 64), (4, 65), (5, 64)])
+def test_width_of_the_sum(sb, ctx, k, trees):
+    rng = np.random.default_rng(10 * trees + k)
+    off, nodes = _forest(sb, rng, trees, 6)
+    x = rng.standard_normal((65, 6)).astype(np.float32)
+    w = rng.random(trees).astype(np.float32)
+    m = sb.BoostedModel.from_arrays(off, nodes, np.zeros(trees + 1, np.int64), [], -0.5, 0 if k == 1 else k, 6,
+                                    objective="multi:softprob" if k > 1 else "reg:squarederror", weights=w, ctx=ctx)
+    nodes = nodes.copy()
+    nodes["leaf_value"] *= np.repeat(w, 7)
+    assert np.array_equal(m.predict_margin(sb.DMatrix(x)), _margins(off, nodes, x, -0.5, k, trees))
