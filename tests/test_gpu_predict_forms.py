@@ -72,3 +72,20 @@ def test_width_of_the_sum(sb, ctx, k, trees):
     nodes = nodes.copy()
     nodes["leaf_value"] *= np.repeat(w, 7)
     assert np.array_equal(m.predict_margin(sb.DMatrix(x)), _margins(off, nodes, x, -0.5, k, trees))
+
+
+@pytest.mark.parametrize("k,trees", [(1, 129), (3, 64), (5, 65), (16, 130), (17, 193)])
+def test_served_outputs(sb, ctx, k, trees):
+    """The serving loop's sum, with more outputs than its blocks have warps."""
+    rng = np.random.default_rng(trees + k)
+    off, nodes = _forest(sb, rng, trees, 6)
+    m = sb.BoostedModel.from_arrays(off, nodes, np.zeros(trees + 1, np.int64), [], -0.5, 0 if k == 1 else k, 6,
+                                    objective="multi:softprob" if k > 1 else "reg:squarederror", ctx=ctx)
+    xs = [rng.standard_normal((n, 6)).astype(np.float32) for n in (1, 33, 70)]
+    srv = sb.Server(m, mem_bytes=64 << 20, n_slots=2)
+    try:
+        tickets = [srv.submit(x) for x in xs]
+        for x, t in zip(xs, tickets):
+            assert np.array_equal(srv.wait(t, timeout_ms=60000)[0], _margins(off, nodes, x, -0.5, k, trees))
+    finally:
+        srv.close()
