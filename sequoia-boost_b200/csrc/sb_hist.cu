@@ -134,7 +134,10 @@ __device__ __forceinline__ uint32_t code_word(uint16_t v, int) { return v; }
 //    without; LANES at 10M rows x 100 features, root level, per launch: 756 us
 //    with a test per row, 486 without). FP32 tests each position: a shared f32
 //    reduction is a compare-and-swap loop, and warps that meet in a lane's
-//    unused word retry (10M rows x 100 features, per launch: 1.78 ms, 0.78 with the test);
+//    unused word retry (10M rows x 100 features, per launch: 1.78 ms, 0.78 with
+//    the test), as do the lanes of one instruction that add the zeros of rows past
+//    the end to row 0's bins (1000 rows x 10 features, whole call 76 us, 63
+//    without those; rounds of 10,000 x 20 337 and 287 us);
 //  - LANES, whose 32 lanes hit 32 banks, needs 8 passes for 4 positions per
 //    lane where TILED's 25 lanes of random bins need 23.
 template <bool FIXED, int KIND, int RL>
@@ -194,7 +197,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
     // flush leaves out (LANES: entry 0 of its column).
     unsigned base[S];
     uint32_t keep[2] = {0, 0};  // code bits that count
-    unsigned pool = 0;          // FP32: the positions that are added
+    unsigned pool = 0;          // FP32: the positions that are added, of rows before the end
 #pragma unroll
     for (int j = 0; j < S; ++j) {
       int f = LANES ? a.slot_feat[pos0 + j] : pos0 + j;
@@ -247,8 +250,8 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
       h = FIXED ? v.x : v.y;
     };
     // The codes of rows [s, s + SUB) of a block. Positions past the part's end
-    // hold row id 0 and a zero pair: their adds change nothing, and no row
-    // needs a test of its own.
+    // hold row id 0 and a zero pair: their adds change nothing, and FIXED needs
+    // no test per row.
     auto load_codes = [&](uint32_t rid, uint32_t s, CW (&bv)[R]) {
 #pragma unroll
       for (int q = 0; q < R; ++q) {
@@ -256,17 +259,18 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
         bv[q] = gather(codes + (uint64_t)id * row_words);
       }
     };
-    auto add_codes = [&](uint32_t g, uint32_t h, uint32_t s, const CW (&bv)[R]) {
+    auto add_codes = [&](uint32_t g, uint32_t h, uint32_t s, uint32_t nr, const CW (&bv)[R]) {
 #pragma unroll
       for (int q = 0; q < R; ++q) {
         const uint32_t src = s + ((uint32_t)q << rl) + (uint32_t)rsub;
         const uint32_t vg = __shfl_sync(0xFFFFFFFFu, g, src);
         const uint32_t vh = __shfl_sync(0xFFFFFFFFu, h, src);
+        const unsigned on = src < nr ? pool : 0u;
 #pragma unroll
         for (int j = 0; j < S; ++j) {
           const uint32_t w = code_word(bv[q], U8 ? 0 : j >> 1) & keep[U8 ? 0 : j >> 1];
           const uint32_t c = U8 ? (w >> (8 * j)) & 0xFFu : (j & 1) ? w >> 16 : w & 0xFFFFu;
-          if (FIXED || (pool >> j & 1)) add_pair<FIXED>(base[j] + 4u * c, hoff, vg, vh);
+          if (FIXED || (on >> j & 1)) add_pair<FIXED>(base[j] + 4u * c, hoff, vg, vh);
         }
       }
     };
@@ -296,10 +300,10 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
 #pragma unroll 1
         for (uint32_t s = 0; s < nr; s += 2 * SUB) {
           load_codes(rid_c, s + SUB, buf1);
-          add_codes(g_c, h_c, s, buf0);
+          add_codes(g_c, h_c, s, nr, buf0);
           const bool inside = s + 2 * SUB < nr;
           load_codes(inside ? rid_c : rid_n, inside ? s + 2 * SUB : 0u, buf0);
-          add_codes(g_c, h_c, s + SUB, buf1);
+          add_codes(g_c, h_c, s + SUB, nr, buf1);
         }
         if (nr_n == 0) break;
         p = pn;
