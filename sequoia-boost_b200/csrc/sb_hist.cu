@@ -1058,6 +1058,17 @@ int hist_time(sb_ctx* ctx, const Ghist* g, float* ms) {
   return rc;
 }
 
+// The CTAs of a launch over m rows by itself (the seam): for few rows one per
+// SM, for more one per 128 (row, tile) units up to the full grid. More CTAs zero
+// and flush more partials than the rows pay for (fixed point, 256 bins, whole call,
+// full grid of 592 / this: 3000 rows x 20 features 115 / 110 us, 50,000 x 30 217 /
+// 204), fewer would put more rows into an f32 partial.
+void seam_grid(sb_ctx* ctx, HistLaunch* L, size_t m) {
+  const size_t units = m * (size_t)L->ntiles, sms = (size_t)ctx->num_sms;
+  L->rows_bound = m;
+  L->rows_per_cta = std::max<size_t>(1, std::min<size_t>(128, units / sms));
+}
+
 // per-node seam helpers (defined in sb_grow.cu)
 int quantize_pairs(sb_ctx* ctx, const float2* d_gp, size_t n, int bits, unsigned long long* d_packed,
                    int* h_shift_g, int* h_shift_h);
@@ -1140,6 +1151,7 @@ int sb_hist_build(sb_ctx* ctx, const sb_ghist* g, const uint32_t* rows, size_t m
   L.ntiles = (int)g->tiles.size();
   L.rows_done = nullptr;
   L.pool_mask = nullptr;
+  seam_grid(ctx, &L, m);
   if (m) SB_TRY(launch_hist(ctx, L));
   const double2* res = d_hist.p;
   if (L.fixed) {
