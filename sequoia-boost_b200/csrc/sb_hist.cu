@@ -768,8 +768,8 @@ size_t smem_budget(const sb_ctx* ctx) {
 
 // Plans the histogram's bin-code layout and feature tiles for one choice
 // (HIST_LAYOUT_TILED, or HIST_LAYOUT_LANES with 1, 2 or 4 code positions per
-// lane and tile). SB_ERR_UNSUPPORTED when a feature's entries do not fit one
-// lane's column.
+// lane and tile). SB_ERR_UNSUPPORTED when a feature's entries do not fit the
+// partial.
 int hist_prepare(sb_ctx* ctx, Ghist* g, HistChoice c) {
   const size_t budget = smem_budget(ctx);
   const size_t F = g->F;
@@ -815,26 +815,64 @@ int hist_prepare(sb_ctx* ctx, Ghist* g, HistChoice c) {
   return SB_OK;
 }
 
+// Device memory that an allocation on the context can still get: what is free
+// on the device and what the pool holds unused.
+static int memory_left(const sb_ctx* ctx, size_t* left) {
+  size_t free_b = 0, total_b = 0;
+  uint64_t reserved = 0, used = 0;
+  cudaMemPool_t pool;
+  SB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  SB_CUDA(cudaDeviceGetDefaultMemPool(&pool, ctx->device));
+  SB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  SB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  *left = free_b + (size_t)(reserved - used);
+  return SB_OK;
+}
+
 // The layout an index takes without timing, or what SB_HIST_LAYOUT ("tiled"
 // or "lanes") in the environment forces. Wide matrices (more than 64 features)
 // of 200k rows and more take LANES with 4 positions per lane where it packs:
 // its adds never meet in a bank. Measured per launch, root / deepest level, us:
 // 10M x 100 x 256 bins 481 / 255 against TILED's 955 / 403; 300k x 100 48 / 80
 // against 71 / 79; 3M x 70 x 64 bins (TILED u8) 141 / 72 against 252 / 115.
+// Two bounds on that:
+//  - at least LANES_MIN_ROWS_PER_BIN rows to a histogram entry. A partial's flush
+//    is dearer than TILED's and there are more tiles of wide features, which few
+//    rows do not pay for (rounds of depth 8, 200k rows, LANES / TILED, ms: 300 x
+//    512 bins, 1.3 rows to an entry, 2.38 / 2.13; 128 x 1024, 1.5, 2.20 / 1.96; 100
+//    x 512, 3.9, 1.17 / 1.07; 80 x 512, 4.9, 1.01 / 1.02; 65 x 512, 6.0, 0.91 /
+//    0.94; 129 x 256, 6.0, 0.78 / 0.86; 100 x 256, 7.8, 0.79 / 0.70);
+//  - its codes take up to five times the memory (256 bytes per row and tile). An
+//    index whose extra codes are more than an eighth of the memory that a TILED
+//    index would leave stays TILED, so that what fits beside such an index fits.
 // Smaller indexes take TILED, the layout that batched jobs share.
+constexpr size_t LANES_MIN_ROWS_PER_BIN = 4, LANES_MEMORY_SHARE = 8;
+constexpr size_t LANES_SMALL_EXTRA = 64 << 20;  // not worth asking the driver (its answer takes some us)
 int hist_default_choice(sb_ctx* ctx, Ghist* g, HistChoice* out) {
   const size_t F = g->F;
   const char* force = std::getenv("SB_HIST_LAYOUT");
   const bool force_lanes = force && std::strcmp(force, "lanes") == 0;
   *out = HistChoice{HIST_LAYOUT_TILED, 0};
-  if (!force_lanes && (force || std::getenv("SB_HIST_ROWS") || F <= 64 || g->n < TUNE_MIN_ROWS)) return SB_OK;
+  if (!force_lanes && (force || std::getenv("SB_HIST_ROWS") || F <= 64 || g->n < TUNE_MIN_ROWS ||
+                       g->n < LANES_MIN_ROWS_PER_BIN * (g->total_bins + F)))
+    return SB_OK;
   const int slots = F <= 32 ? 1 : (F <= 64 ? 2 : 4);
   std::vector<std::vector<LanePlace>> places;
   const std::vector<FeatureTile> keep = g->tiles;
   const bool ok = plan_lanes(g, smem_budget(ctx), slots, &places) == SB_OK;
+  const size_t lanes_row = g->tiles.size() * 32 * slots * 2;
   g->tiles = keep;
   SB_REQUIRE(ok || !force_lanes, SB_ERR_UNSUPPORTED, "SB_HIST_LAYOUT=lanes: a feature has too many bins");
-  if (ok) *out = HistChoice{HIST_LAYOUT_LANES, slots};
+  if (!ok) return SB_OK;
+  const size_t tiled_row = (F + 7) / 8 * 8 * (g->max_feature_bins <= 255 ? 1 : 2);
+  const size_t extra = lanes_row > tiled_row ? g->n * (lanes_row - tiled_row) : 0;
+  if (!force_lanes && extra > LANES_SMALL_EXTRA) {
+    size_t left = 0;
+    SB_TRY(memory_left(ctx, &left));
+    const size_t tiled = g->n * (tiled_row + 2 * F);  // with the feature-major bins
+    if (left < tiled || (left - tiled) / LANES_MEMORY_SHARE < extra) return SB_OK;
+  }
+  *out = HistChoice{HIST_LAYOUT_LANES, slots};
   return SB_OK;
 }
 
