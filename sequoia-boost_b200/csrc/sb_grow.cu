@@ -2399,8 +2399,6 @@ int quantize_pairs(sb_ctx* ctx, const float2* d_gp, size_t n, int bits, unsigned
 
 namespace {
 
-// Objective::base_margin / prob_to_margin with TrainingParams::base_score
-// (learner/train.rs:203-210) from host labels and weights.
 // Sum, sum of magnitudes and count of non-integers of n labels, into out[3].
 __global__ void __launch_bounds__(256) k_label_stats(const float* __restrict__ y, size_t n, double* __restrict__ out) {
   double v[3] = {0.0, 0.0, 0.0};
@@ -2422,11 +2420,16 @@ __global__ void k_fill(float* __restrict__ p, size_t n, float v) {
 // The labels' sum where every partial sum is an integer below 2^53: exact in
 // f64, so the device's sum in any order is the sequential one (class labels,
 // counts). A long vector's sequential additions take a nanosecond each on the
-// host (10M labels 10 ms, this 0.05 ms). *exact = false otherwise.
-constexpr size_t LABEL_SUM_MIN = 65536;
-int label_sum(sb_ctx* ctx, const float* d_labels, size_t n, double* sum, bool* exact) {
+// host (10M labels 10 ms, this 0.05 ms and more); the launch and the wait take as
+// long as 100,000 of them. *exact = false otherwise, and without a launch where
+// one of the first labels is no integer: real labels would pay for both (a booster
+// over 100,000 of them 0.22 ms, 0.26 with the launch).
+constexpr size_t LABEL_SUM_MIN = 131072, LABEL_SUM_LOOK = 64;
+int label_sum(sb_ctx* ctx, const float* labels, const float* d_labels, size_t n, double* sum, bool* exact) {
   *exact = false;
   if (n < LABEL_SUM_MIN) return SB_OK;
+  for (size_t i = 0; i < LABEL_SUM_LOOK; ++i)
+    if (labels[i] != std::rint(labels[i])) return SB_OK;
   DBuf<double> d;
   SB_TRY(d.alloc_zero(ctx, 3));
   const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 8);
@@ -2439,7 +2442,9 @@ int label_sum(sb_ctx* ctx, const float* d_labels, size_t n, double* sum, bool* e
   return SB_OK;
 }
 
-// known_sum: the labels' sum where it is known already, or null.
+// Objective::base_margin / prob_to_margin with TrainingParams::base_score
+// (learner/train.rs:203-210) from host labels and weights. known_sum: the
+// labels' sum where it is known already, or null.
 float base_margin_of(const sb_train_params* p, const float* labels, const float* weights, size_t n, int K,
                      const double* known_sum = nullptr) {
   float base;
@@ -3566,7 +3571,7 @@ int sb_booster_create(sb_ctx* ctx, const sb_ghist* g, const sb_train_params* p, 
   }
   double sum = 0.0;
   bool exact = false;
-  if (K == 1 && !p->has_base_score && !weights) SB_TRY(label_sum(ctx, b->d_labels.p, n, &sum, &exact));
+  if (K == 1 && !p->has_base_score && !weights) SB_TRY(label_sum(ctx, labels, b->d_labels.p, n, &sum, &exact));
   const float base = base_margin_of(p, labels, weights, n, K, exact ? &sum : nullptr);
   b->base_score = base;
   if (base_margin) {  // init_margin, train.rs:496-511

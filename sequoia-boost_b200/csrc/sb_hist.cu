@@ -847,7 +847,7 @@ static int memory_left(const sb_ctx* ctx, size_t* left) {
 //    index would leave stays TILED, so that what fits beside such an index fits.
 // Smaller indexes take TILED, the layout that batched jobs share.
 constexpr size_t LANES_MIN_ROWS_PER_BIN = 4, LANES_MEMORY_SHARE = 8;
-constexpr size_t LANES_SMALL_EXTRA = 64 << 20;  // not worth asking the driver (its answer takes some us)
+constexpr size_t LANES_SMALL_EXTRA = 256 << 20;  // not worth asking the driver: its answer takes 0.09 ms
 int hist_default_choice(sb_ctx* ctx, Ghist* g, HistChoice* out) {
   const size_t F = g->F;
   const char* force = std::getenv("SB_HIST_LAYOUT");
