@@ -196,9 +196,10 @@ int sb_ghist_bins(const sb_ghist* g, uint16_t* local_bins);
  * u8 or u16 row-major codes, n_rows rows of `row_stride` codes.
  * layout: 0 = TILED, 1 = LANES; code_bytes: 1 when the layout is TILED and
  * every feature has at most 255 bins (then feature f's code sits at position
- * f: its local bin, or its bin count when missing), else 2 (tile-relative
- * histogram entries); rows_per_instruction: rows one warp instruction of the
- * histogram kernel covers. Any pointer may be NULL. */
+ * f: its local bin, or its bin count when missing), else 2 (TILED: the entry of
+ * the feature tile's histogram; LANES: the word of the tile's shared partial);
+ * rows_per_instruction: rows one warp instruction of the histogram kernel
+ * covers. Any pointer may be NULL. */
 int sb_ghist_layout(const sb_ghist* g, int* layout, int* code_bytes, size_t* row_stride,
                     int* rows_per_instruction);
 /* Copies the n_rows * row_stride codes (code_bytes each) to `codes` (host). */

@@ -15,7 +15,7 @@
 // One boosting round is a fixed sequence of kernels whose work sizes live in
 // device memory (no host round trip inside a round):
 //   k_gradient -> k_round_prep -> [k_quantize] -> root histograms ->
-//   per level d: k_eval -> k_assign -> k_partition -> k_plan -> histograms
+//   per level d: [k_eval_scan ->] k_eval -> k_assign -> k_partition -> k_plan -> histograms
 //   -> k_round_end.
 // All frontier nodes of all K class trees are processed by each launch.
 #include <algorithm>
@@ -83,9 +83,9 @@ struct BState {
   int* prev_count;          // [K] frontier nodes expanded by the last k_assign
   size_t n, Fp;
   // binned data
-  const uint16_t* bins;      // tile-relative codes, row-major (u16 codes)
+  const uint16_t* bins;      // row-major codes (u16) as the histogram kernel reads them
   const uint8_t* bins8;      // the same with u8 codes (bins null)
-  const uint16_t* bins_col;  // the same, feature-major
+  const uint16_t* bins_col;  // local bins, feature-major
   const int* fbase;          // code of local bin 0, per feature
   const int* fmiss;          // code of a missing entry, per feature
   const int* rpos;           // row-major codes: position, code of local bin 0 and

@@ -3,14 +3,14 @@
 //
 // Each job gets its own binned matrix and device booster (train(), learner/
 // train.rs:107-113, per job), set up by a few host threads at once, jobs
-// spread round-robin over a pool of streams. Depthwise jobs of one precision
-// and one row grouping then train in batches: every round of a batch is one
-// launch per kernel step for all its jobs (their grids laid end to end, each
-// block running its job's state), recorded once as a CUDA graph and
+// spread round-robin over a pool of streams. Depthwise jobs of one precision,
+// row grouping, code width and CTA size then train in batches: every round of a
+// batch is one launch per kernel step for all its jobs (their grids laid end to
+// end, each block running its job's state), recorded once as a CUDA graph and
 // replayed. Jobs are sorted by size into up to 8 batches of similar jobs that
 // run at once on their own streams. The jobs that cannot share launches
-// (lossguide, eval sets, the LANES layout) are issued round r of every job
-// before round r + 1 of any over the pool.
+// (lossguide, eval sets, the LANES layout, the only one of its kind) are issued
+// round r of every job before round r + 1 of any over the pool.
 #include <algorithm>
 #include <thread>
 #include <vector>

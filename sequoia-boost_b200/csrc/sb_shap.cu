@@ -638,8 +638,7 @@ k_shap_table(ShapTabDev P, const float* __restrict__ X, size_t n, int F, float m
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             if (4 * j + q < MAXD && 4 * j + q < hd[u].y) {
-              if (TPR == 1) pr[fc[u][4 * j + q] * R] += vv[q];
-              else atomicAdd(pr + fc[u][4 * j + q] * R, vv[q]);  // the row's other threads add too
+              atomicAdd(pr + fc[u][4 * j + q] * R, vv[q]);  // the row's other threads add too
             }
         }
       }
@@ -1182,7 +1181,7 @@ int contribs_bias(sb_model* m, std::vector<double>* bias) {
   SB_TRY(shap_prepare(m));
   const int K = m->num_class >= 2 ? m->num_class : 1;
   bias->assign(K, (double)m->base_score);
-  for (size_t t = 0; t < m->trees.size(); ++t) (*bias)[t % K] += node_mean_value(m->trees[t], 0);
+  for (size_t t = 0; t < m->trees.size(); ++t) (*bias)[t % K] += m->dev.tree_mean[t];
   return SB_OK;
 }
 
