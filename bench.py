@@ -138,16 +138,19 @@ def peaks():
         return 6650.0, "fallback"
 
 
-def traffic_per_launch():
-    """dram read+write bytes of one histogram launch, from the committed ncu
-    summary of the same kernel (scaled to this workload), or None."""
+def traffic_per_launch(layout, bytes_per_launch):
+    """dram read+write bytes of one histogram launch: the algorithmic bytes
+    times the ratio of the committed ncu summary, or None where that summary
+    was taken with codes of another form (`layout`, GHistIndex.layout())."""
     path = os.path.join(ROOT, "profiles", "k_hist_traffic.json")
     try:
         with open(path) as fh:
             d = json.load(fh)
-        return d
     except (OSError, ValueError):
         return None
+    if d.get("layout") != layout:
+        return None
+    return d["traffic_over_algorithmic"] * bytes_per_launch
 
 
 def logloss(margin, y):
@@ -585,13 +588,13 @@ def main():
     b.set_timing(False)
     peak, peak_kind = peaks()
     achieved = st["hist_bytes"] / (st["hist_ms"] / 1e3) / 1e9 if st["hist_ms"] > 0 else None
-    tr = traffic_per_launch()
+    bytes_per_launch = st["hist_bytes"] / max(st["hist_launches"], 1)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": None if achieved is None else achieved / peak, "peak_kind": peak_kind,
-                "traffic": None if tr is None else tr.get("bytes_per_launch"),
+                "traffic": traffic_per_launch(gh.layout(), bytes_per_launch),
                 "kernel": f"k_hist<{'fixed' if args.precision == 'fixed' else 'fp32'}>",
                 "launches_timed": st["hist_launches"],
-                "bytes_per_launch": st["hist_bytes"] / max(st["hist_launches"], 1),
+                "bytes_per_launch": bytes_per_launch,
                 "ms_per_launch": st["hist_ms"] / max(st["hist_launches"], 1),
                 "hist_share_of_round": st["hist_ms"] / st["round_ms"] if st["round_ms"] else None}
     rounds_total = args.warmup + args.steps + min(args.steps, 5)
