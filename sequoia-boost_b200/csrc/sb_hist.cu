@@ -1096,12 +1096,14 @@ int hist_time(sb_ctx* ctx, const Ghist* g, float* ms) {
   return rc;
 }
 
-// The CTAs of a launch over m rows by itself (the seam): for few rows one per
-// SM, for more one per 128 (row, tile) units up to the full grid. More CTAs zero
-// and flush more partials than the rows pay for (fixed point, 256 bins, whole call,
-// full grid of 592 / this: 3000 rows x 20 features 115 / 110 us, 50,000 x 30 217 /
-// 204), fewer would put more rows into an f32 partial.
-void seam_grid(sb_ctx* ctx, HistLaunch* L, size_t m) {
+// The CTAs of a fixed-point launch over m rows by itself (the seam): for few
+// rows one per SM, for more one per 128 (row, tile) units up to the full grid.
+// More CTAs zero and flush more partials than the rows pay for (256 bins, whole
+// call, full grid of 592 / this: 3000 rows x 20 features 115 / 110 us, 50,000 x 30
+// 217 / 204). FP32 keeps the full grid: fewer CTAs put more rows into an f32
+// partial (1000 rows x 8 features: error against 64 bits 1.3e-9, 5.6e-9 with 148).
+static void seam_grid(sb_ctx* ctx, HistLaunch* L, size_t m) {
+  if (!L->fixed) return;
   const size_t units = m * (size_t)L->ntiles, sms = (size_t)ctx->num_sms;
   L->rows_bound = m;
   L->rows_per_cta = std::max<size_t>(1, std::min<size_t>(128, units / sms));

@@ -329,7 +329,6 @@ int hist_time(sb_ctx* ctx, const Ghist* g, float* ms);
 int launch_hist(sb_ctx* ctx, const HistLaunch& L);
 int launch_zero_items(sb_ctx* ctx, const HistLaunch& L);  // before launch_hist: zeroes L's items, fills L.parts
 int hist_grid(sb_ctx* ctx, const Ghist* g, size_t rows_bound, size_t rows_per_cta);
-void seam_grid(sb_ctx* ctx, HistLaunch* L, size_t m);  // sets L's grid for a launch over m rows by itself
 // Depthwise boosters that can share batched round launches (no lossguide,
 // external gradients, timing, eval sets or row -> leaf output; TILED index).
 bool booster_batchable(const sb_booster* b);

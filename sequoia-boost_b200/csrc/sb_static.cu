@@ -141,7 +141,6 @@ int sb_hist_build_static(sb_ctx* ctx, const sb_ghist* g, const uint32_t* d_rows,
     L.ntiles = (int)g->tiles.size();
     L.rows_done = nullptr;
     L.pool_mask = nullptr;
-    seam_grid(ctx, &L, m);
     SB_TRY(launch_hist(ctx, L));
   }
   // the present bins (global bin order); the missing bins stay in scratch
