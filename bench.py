@@ -83,7 +83,7 @@ def config_of(args, n):
     return {"workload": f"binary_mixed {n} x 100 (binary:logistic, depth 8, max_bin 256, eta 0.05, "
                         "subsample 0.8, colsample_bytree 0.8)",
             "n_rows": n, "n_features": 100, "rounds_per_step": 1, "precision": args.precision,
-            "l2": "inputs larger than L2 (ELLPACK 2 B/entry = 2.1 GB at 10M rows)",
+            "l2": "inputs larger than L2 (row codes of 256 B a row = 2.6 GB at 10M rows)",
             "parallelism": f"replicas x{args.gpus}"}
 
 
