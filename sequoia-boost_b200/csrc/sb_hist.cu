@@ -148,7 +148,7 @@ __device__ __forceinline__ void hist_body(const HistDev& a, unsigned bx, unsigne
   constexpr int R = rl == 3 ? 2 : S == 4 ? 4 : 8;  // steps per sub-batch
   constexpr uint32_t SUB = (uint32_t)R << rl;      // rows per sub-batch: two or more fill a block of 32
   using CW = typename Codes<KIND>::T;
-  extern __shared__ unsigned long long sh_u64[];
+  extern __shared__ __align__(16) unsigned long long sh_u64[];  // zeroed 16 bytes at a time
   unsigned* sh_g = reinterpret_cast<unsigned*>(sh_u64);
   __shared__ double s_tot_d[2];
   __shared__ unsigned long long s_tot_u[2];
