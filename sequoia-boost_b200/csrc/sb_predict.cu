@@ -113,7 +113,7 @@ __device__ __forceinline__ float margin_start(const MarginStart& m, size_t r, in
 }
 
 // Margins in two phases. Phase 1: the leaf value of every (row, tree),
-// tree-major. A block takes 2^lr >= min(n, 32) rows and a tree per remaining
+// tree-major. A block takes 2^lr rows, up to 32, and a tree per remaining
 // thread, so that all trees of a small request are walked at once: its time is
 // one tree's chain of dependent loads. With many rows a thread takes up to 8
 // trees and the block's rows are staged in shared memory (read row by row from
@@ -252,10 +252,13 @@ struct LeafPlan {
 // memory at any size, since their walk leaves L1 to the rows (4096 rows x 100
 // features, 500 trees of depth 8 with categorical splits: 464 staged, 362 not).
 // Without staging a thread takes one tree: more of them only leave an uneven
-// last wave (the same call: 362 at up to 8 trees, 301 at one).
+// last wave (the same call: 362 at up to 8 trees, 301 at one). A warp has one
+// tree of 16-byte nodes however few the rows: lanes wait for one another's
+// category lists, and trees in one warp meet theirs at different steps (one row,
+// 100 trees of lists of some 100 categories: 128 with 32 trees to a warp, 68).
 LeafPlan leaf_plan(size_t n, size_t F, size_t limit, bool compact, int num_sms) {
   LeafPlan p{0, 0, 1, 0};
-  while (p.lr < 5 && ((size_t)1 << p.lr) < n) ++p.lr;
+  while (p.lr < 5 && (!compact || ((size_t)1 << p.lr) < n)) ++p.lr;
   // one tree per thread while all fit the chip at once, up to 8
   const size_t pairs = n * limit, chip = (size_t)num_sms * 2048;
   const int many = (int)std::max<size_t>(1, std::min<size_t>(8, pairs / chip));
